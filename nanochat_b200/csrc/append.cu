@@ -1,7 +1,8 @@
 // Kernel (a): fused RoPE + QK rms-norm + scale + KV append, bit-exact against the eager bf16 path.
 //
-// One half-warp (16 lanes x 8 bf16 = one 256-byte head row, 16-byte loads and stores) handles
-// one (row b, token t, head) of q, k or v.  The arithmetic reproduces, rounding for rounding,
+// One half-warp handles head rows of one token of q, k or v: lane j of its 16 holds channels 4j .. 4j + 3 and
+// 64 + 4j .. 64 + 4j + 3, the two sides of its rotation pairs (8-byte loads and stores, 128 contiguous bytes per
+// half-warp), so the rotation crosses no lanes.  The arithmetic reproduces, rounding for rounding,
 // the reference's op sequence on bf16 tensors:
 //   apply_rotary_emb (gpt.py:57-63):  y1 = bf16(bf16(x1*cos) + bf16(x2*sin))
 //                                     y2 = bf16(bf16(x1*(-sin)) + bf16(x2*cos))
@@ -38,84 +39,70 @@ struct AppendParams {
     // distance between the tokens of q_in / k_in / v_in in 16-byte units (heads of a token are packed); lets the
     // three be column slices of one projection output
     long long q_stride, k_stride, v_stride;
+    int per_tok;  // half-warps per token
 };
 
-__device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8]) {
+__device__ __forceinline__ void unpack4(const uint2 &v, float (&f)[4]) {
     f[0] = bf16lo(v.x); f[1] = bf16hi(v.x);
     f[2] = bf16lo(v.y); f[3] = bf16hi(v.y);
-    f[4] = bf16lo(v.z); f[5] = bf16hi(v.z);
-    f[6] = bf16lo(v.w); f[7] = bf16hi(v.w);
 }
-__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
-    uint4 v;
-    v.x = pack_bf16x2(f[0], f[1]);
-    v.y = pack_bf16x2(f[2], f[3]);
-    v.z = pack_bf16x2(f[4], f[5]);
-    v.w = pack_bf16x2(f[6], f[7]);
-    return v;
+__device__ __forceinline__ uint2 pack4(const float (&f)[4]) {
+    return make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
 }
-__device__ __forceinline__ uint4 shfl_xor_u4(const uint4 &v, int mask) {
-    uint4 r;
-    r.x = __shfl_xor_sync(0xffffffffu, v.x, mask);
-    r.y = __shfl_xor_sync(0xffffffffu, v.y, mask);
-    r.z = __shfl_xor_sync(0xffffffffu, v.z, mask);
-    r.w = __shfl_xor_sync(0xffffffffu, v.w, mask);
-    return r;
+// bf16(bf16(a * c) + bf16(b * s)) on four elements
+__device__ __forceinline__ void rotate4(const float (&a)[4], const float (&c)[4], const float (&b)[4], const float (&s)[4], float (&y)[4]) {
+    float t1[4], t2[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        t1[i] = __fmul_rn(a[i], c[i]);
+        t2[i] = __fmul_rn(b[i], s[i]);
+    }
+    unpack4(pack4(t1), t1);
+    unpack4(pack4(t2), t2);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[i] = __fadd_rn(t1[i], t2[i]);
+    unpack4(pack4(y), y);
+}
+__device__ __forceinline__ float squares4(const float (&y)[4]) {
+    float e = __fmul_rn(y[0], y[0]);
+    e = __fmaf_rn(y[1], y[1], e);
+    e = __fmaf_rn(y[2], y[2], e);
+    return __fmaf_rn(y[3], y[3], e);
 }
 
-// RoPE -> rms-norm -> scale on one 128-wide head row held 8 elements per lane by 16 lanes.
-// `j` is the lane's index within its half-warp (0..15); all 32 lanes must call this.
-__device__ __forceinline__ uint4 rope_norm_scale(const uint4 &xin, const uint4 &cosv,
-                                                 const uint4 &sinv, int j, float qk_scale,
-                                                 float eps) {
-    float own[8], oth[8], c[8], s[8], y[8];
-    uint4 partner = shfl_xor_u4(xin, 8);  // channel i <-> i + 64
-    unpack8(xin, own);
-    unpack8(partner, oth);
-    unpack8(cosv, c);
-    unpack8(sinv, s);
-    const bool first_half = j < 8;
+// RoPE -> rms-norm -> scale on a 128-wide head row held by 16 lanes; all 32 lanes of a warp must call this.
+__device__ __forceinline__ void rope_norm_scale(uint2 &lo, uint2 &hi, const float (&c)[4], const float (&s)[4], float qk_scale, float eps) {
+    float x1[4], x2[4], y1[4], y2[4], neg_s[4];
+    unpack4(lo, x1);
+    unpack4(hi, x2);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if (first_half) {  // own = x1, oth = x2
-            float t1 = round_bf16(__fmul_rn(own[i], c[i]));
-            float t2 = round_bf16(__fmul_rn(oth[i], s[i]));
-            y[i] = round_bf16(__fadd_rn(t1, t2));
-        } else {  // own = x2, oth = x1
-            float t3 = round_bf16(__fmul_rn(oth[i], -s[i]));
-            float t4 = round_bf16(__fmul_rn(own[i], c[i]));
-            y[i] = round_bf16(__fadd_rn(t3, t4));
-        }
-    }
-    // sum of squares: two "virtual lanes" of 4 consecutive elements per real lane
-    float e0 = __fmul_rn(y[0], y[0]);
-    e0 = __fmaf_rn(y[1], y[1], e0);
-    e0 = __fmaf_rn(y[2], y[2], e0);
-    e0 = __fmaf_rn(y[3], y[3], e0);
-    float e1 = __fmul_rn(y[4], y[4]);
-    e1 = __fmaf_rn(y[5], y[5], e1);
-    e1 = __fmaf_rn(y[6], y[6], e1);
-    e1 = __fmaf_rn(y[7], y[7], e1);
-    // virtual shuffle-down tree with offsets 16, 8, 4, 2 (= real-lane offsets 8, 4, 2, 1), then 1
+    for (int i = 0; i < 4; ++i) neg_s[i] = -s[i];
+    rotate4(x1, c, x2, s, y1);
+    rotate4(x1, neg_s, x2, c, y2);
+    // Offset 16 of the tree joins lanes that one thread holds here.  Every level adds the same pairs as the
+    // shuffle-down does for its lane 0, whichever lane of the butterfly looks at it (a sum of two commutes).
+    float e = __fadd_rn(squares4(y1), squares4(y2));
 #pragma unroll
-    for (int off = 8; off >= 1; off >>= 1) {
-        float o0 = __shfl_down_sync(0xffffffffu, e0, off, 16);
-        float o1 = __shfl_down_sync(0xffffffffu, e1, off, 16);
-        e0 = __fadd_rn(e0, o0);
-        e1 = __fadd_rn(e1, o1);
-    }
-    float total = __fadd_rn(e0, e1);
-    total = __shfl_sync(0xffffffffu, total, 0, 16);
-    const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(total, 128.0f), eps));
-    float o[8];
+    for (int off = 8; off >= 1; off >>= 1) e = __fadd_rn(e, __shfl_xor_sync(0xffffffffu, e, off));
+    const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(e, 128.0f), eps));
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        float z = round_bf16(__fmul_rn(y[i], rstd));
-        o[i] = __fmul_rn(z, qk_scale);  // pack8 applies the final bf16 rounding
+    for (int i = 0; i < 4; ++i) {
+        y1[i] = __fmul_rn(y1[i], rstd);
+        y2[i] = __fmul_rn(y2[i], rstd);
     }
-    return pack8(o);
+    unpack4(pack4(y1), y1);
+    unpack4(pack4(y2), y2);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // pack4 applies the final bf16 rounding
+        y1[i] = __fmul_rn(y1[i], qk_scale);
+        y2[i] = __fmul_rn(y2[i], qk_scale);
+    }
+    lo = pack4(y1);
+    hi = pack4(y2);
 }
 
+// NB: head rows a half-warp takes, all of one token and loaded together (rows first, first + per_tok, ...).
+template <int NB>
 __global__ void __launch_bounds__(256) append_rope_norm_kernel(const AppendParams p) {
     // Programmatic dependent launch: this grid may have been scheduled while its predecessor was
     // still running; its inputs come from that predecessor, so wait before touching anything.
@@ -123,81 +110,85 @@ __global__ void __launch_bounds__(256) append_rope_norm_kernel(const AppendParam
     // reads only cache_seqlens and older cache rows until it has itself waited for this grid.
     pdl_launch_dependents();
     pdl_wait_prior_grids();
-    const int lane = threadIdx.x & 31;
-    const int j = lane & 15;
-    const int heads_per_tok = (p.q_in ? p.Hq : 0) + 2 * p.Hkv;
-    const int q_heads = p.q_in ? p.Hq : 0;
-    const long long total_rows = (long long)p.B * p.T_new * heads_per_tok;
-    const long long n_half_warps = ((long long)gridDim.x * blockDim.x) >> 4;
-    long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-    // rows are padded to an even count per iteration so both half-warps stay convergent
-    const long long padded = (total_rows + 1) & ~1LL;
-    for (; row < padded; row += n_half_warps) {
-        const bool live = row < total_rows;
-        const long long r = live ? row : total_rows - 1;
-        const int slot = (int)(r % heads_per_tok);
-        const long long bt = r / heads_per_tok;
-        const int t = (int)(bt % p.T_new);
-        const int b = (int)(bt / p.T_new);
-        // kind: 0 = q head, 1 = k head, 2 = v head.  The two half-warps of a warp may hold
-        // different kinds, so the transform (which shuffles across the warp) runs unconditionally
-        // and its result is selected afterwards.
+    const int j = threadIdx.x & 15;
+    const int q_heads = p.q_in ? p.Hq : 0, heads_per_tok = q_heads + 2 * p.Hkv;
+    const unsigned half_warp = (blockIdx.x * 256u + threadIdx.x) >> 4, n_tok = (unsigned)p.B * (unsigned)p.T_new;
+    unsigned tok = half_warp / (unsigned)p.per_tok;
+    const int first = (int)(half_warp - tok * (unsigned)p.per_tok);
+    const bool live = tok < n_tok;
+    if (!live) tok = n_tok - 1;  // stays for the shuffles
+    const int b = (int)(tok / (unsigned)p.T_new), t = (int)(tok - (unsigned)b * (unsigned)p.T_new);
+    // the input rows do not depend on the row's length: their loads go out together with the
+    // length's, one round trip ahead of the table rows that do
+    uint2 lo[NB], hi[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int slot = first + i * p.per_tok;
+        lo[i] = hi[i] = make_uint2(0, 0);
+        if (!live || slot >= heads_per_tok) continue;
+        // kind: 0 = q head, 1 = k head, 2 = v head
         const int kind = slot < q_heads ? 0 : (slot < q_heads + p.Hkv ? 1 : 2);
-        const int h = kind == 0 ? slot : (kind == 1 ? slot - q_heads : slot - q_heads - p.Hkv);
-        const bool transform = kind == 0 || (kind == 1 && p.transform_k);
-        const uint4 *src = kind == 0 ? p.q_in : (kind == 1 ? p.k_in : p.v_in);
-        const long long src_idx = (bt * (kind == 0 ? p.Hq : p.Hkv) + h) * 16 + j;  // packed: where q_out goes
-        const long long in_idx = bt * (kind == 0 ? p.q_stride : (kind == 1 ? p.k_stride : p.v_stride)) + h * 16 + j;
-        // the input row does not depend on the row's length: its load goes out together with the
-        // length's, one round trip ahead of the table rows that do
-        uint4 x = make_uint4(0, 0, 0, 0);
-        if (live) x = src[in_idx];
-        const int len = p.cache_seqlens[b];          // sequence position of token 0 (drives RoPE)
-        int wslot = p.write_slots ? p.write_slots[b] : len;  // cache index of token 0
-        if (p.split.block > 0 && len >= 0)
-            wslot = (len / p.split.block) % p.split.world == p.split.rank
-                        ? owned_below(len, p.split.world, p.split.rank, p.split.block) : -1;
-        const int pos = len + t;
-        bool ok = live;
-        if (len < 0 || wslot < -1) {
-            if (live && j == 0 && slot == 0 && t == 0) atomicOr(p.status, (int)NCKV_ST_BAD_SEQLEN);
-            ok = false;
-        } else if ((wslot >= 0 && wslot + p.T_new > p.T_max) || (p.rope_len > 0 && len + p.T_new > p.rope_len)) {
-            if (live && j == 0 && slot == 0 && t == 0) atomicOr(p.status, (int)NCKV_ST_OVERFLOW);
-            ok = false;
-        }
-        const bool write_kv = ok && wslot >= 0;  // -1: this row's token belongs to another shard
-        const int safe_pos = ok ? pos : 0;
-        uint4 cv = make_uint4(0, 0, 0, 0), sv = cv;
-        if (!ok) x = cv;
-        if (ok && transform) {
-            cv = p.cos[(long long)safe_pos * 8 + (j & 7)];
-            sv = p.sin[(long long)safe_pos * 8 + (j & 7)];
-        }
-        uint4 o = rope_norm_scale(x, cv, sv, j, p.qk_scale, p.eps);
-        if (!transform) o = x;
-        if (ok) {
-            if (kind == 0) {
-                p.q_out[src_idx] = o;
-            } else if (write_kv) {
-                __nv_bfloat16 *cache = kind == 1 ? p.k_cache : p.v_cache;
-                long long outer = b, tok = wslot + t;
-                if (p.block_table) {  // row -> page
-                    const int idx = (int)(tok / p.page_tokens);
-                    tok -= (long long)idx * p.page_tokens;
-                    outer = p.block_table[(long long)b * p.max_pages + idx];
-                    if (outer < 0 || outer >= p.n_pages) {
-                        if (j == 0 && h == 0 && kind == 1) atomicOr(p.status, (int)NCKV_ST_BAD_PAGE);
-                        outer = -1;
-                    }
-                }
-                if (outer >= 0) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(cache + outer * p.cache_batch_stride +
-                                                           tok * p.cache_token_stride + (long long)h * NCKV_D);
-                    dst[j] = o;
-                }
+        const int h = slot - (kind == 0 ? 0 : (kind == 1 ? q_heads : q_heads + p.Hkv));
+        const uint4 *row = (kind == 0 ? p.q_in : (kind == 1 ? p.k_in : p.v_in)) +
+                           tok * (kind == 0 ? p.q_stride : (kind == 1 ? p.k_stride : p.v_stride)) + h * 16;
+        lo[i] = reinterpret_cast<const uint2 *>(row)[j];
+        hi[i] = reinterpret_cast<const uint2 *>(row)[16 + j];
+    }
+    const int len = p.cache_seqlens[b];          // sequence position of token 0 (drives RoPE)
+    int wslot = p.write_slots ? p.write_slots[b] : len;  // cache index of token 0
+    if (p.split.block > 0 && len >= 0)
+        wslot = (len / p.split.block) % p.split.world == p.split.rank
+                    ? owned_below(len, p.split.world, p.split.rank, p.split.block) : -1;
+    bool ok = live;
+    if (len < 0 || wslot < -1) {
+        if (live && j == 0 && first == 0 && t == 0) atomicOr(p.status, (int)NCKV_ST_BAD_SEQLEN);
+        ok = false;
+    } else if ((wslot >= 0 && wslot + p.T_new > p.T_max) || (p.rope_len > 0 && len + p.T_new > p.rope_len)) {
+        if (live && j == 0 && first == 0 && t == 0) atomicOr(p.status, (int)NCKV_ST_OVERFLOW);
+        ok = false;
+    }
+    const bool write_kv = ok && wslot >= 0;  // -1: this row's token belongs to another shard
+    float c[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
+    if (ok && p.rope_len > 0) {
+        const long long at = (long long)(len + t) * 16 + j;
+        unpack4(reinterpret_cast<const uint2 *>(p.cos)[at], c);
+        unpack4(reinterpret_cast<const uint2 *>(p.sin)[at], s);
+    }
+    long long dst_off = 0;  // of the token's heads in the caches
+    bool in_cache = write_kv;
+    if (write_kv) {
+        long long outer = b, at = wslot + t;
+        if (p.block_table) {  // row -> page
+            const int idx = (int)(at / p.page_tokens);
+            at -= (long long)idx * p.page_tokens;
+            outer = p.block_table[(long long)b * p.max_pages + idx];
+            if (outer < 0 || outer >= p.n_pages) {
+                if (j == 0 && first == 0) atomicOr(p.status, (int)NCKV_ST_BAD_PAGE);
+                in_cache = false;
             }
         }
+        dst_off = outer * p.cache_batch_stride + at * p.cache_token_stride;
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int slot = first + i * p.per_tok;
+        const int kind = slot < q_heads ? 0 : (slot < q_heads + p.Hkv ? 1 : 2);
+        const int h = slot - (kind == 0 ? 0 : (kind == 1 ? q_heads : q_heads + p.Hkv));
+        const bool transform = kind == 0 || (kind == 1 && p.transform_k);
+        // the two half-warps may hold different kinds, and the transform shuffles across the warp
+        if (__any_sync(0xffffffffu, transform)) {
+            uint2 a = lo[i], d = hi[i];
+            rope_norm_scale(a, d, c, s, p.qk_scale, p.eps);
+            if (transform) {
+                lo[i] = a;
+                hi[i] = d;
+            }
+        }
+        if (slot >= heads_per_tok || !ok || (kind != 0 && !in_cache)) continue;
+        uint2 *dst = kind == 0 ? reinterpret_cast<uint2 *>(p.q_out + ((long long)tok * p.Hq + h) * 16)
+                               : reinterpret_cast<uint2 *>((kind == 1 ? p.k_cache : p.v_cache) + dst_off + (long long)h * NCKV_D);
+        dst[j] = lo[i];
+        dst[16 + j] = hi[i];
     }
 }
 
@@ -232,16 +223,23 @@ static int check_common(const void *k_in, const void *v_in, void *k_cache, void 
     return NCKV_OK;
 }
 
-static int launch_append(const AppendParams &p, cudaStream_t stream) {
+// Rows per half-warp.  Few rows (a decode step): one each, the shortest chain from the input to the store.  From
+// APPEND_WIDE_ROWS head rows on the chip is full either way, and four rows share the index arithmetic and the
+// token's table row.
+constexpr long long APPEND_WIDE_ROWS = 32768;
+
+static int launch_append(AppendParams p, cudaStream_t stream) {
     const int heads_per_tok = (p.q_in ? p.Hq : 0) + 2 * p.Hkv;
-    const long long rows = (long long)p.B * p.T_new * heads_per_tok;
-    const int threads = 256;                                   // 16 head rows per CTA
-    long long blocks = (rows + 15) / 16;
-    const long long cap = (long long)sm_count() * 8 * 4;       // grid-stride beyond this
-    if (blocks > cap) blocks = cap;
+    const bool wide = (long long)p.B * p.T_new * heads_per_tok >= APPEND_WIDE_ROWS;
+    p.per_tok = wide ? (heads_per_tok + 3) / 4 : heads_per_tok;
+    const long long half_warps = (long long)p.B * p.T_new * p.per_tok;
+    if (half_warps > 0xfffffff0LL) {
+        set_error("append: B=%d x T_new=%d tokens are too many for one launch", p.B, p.T_new);
+        return NCKV_E_UNSUPPORTED;
+    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(threads);
+    cfg.gridDim = dim3((unsigned)((half_warps + 15) / 16));
+    cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -249,7 +247,7 @@ static int launch_append(const AppendParams &p, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    NCKV_CUDA_CHECK(cudaLaunchKernelEx(&cfg, append_rope_norm_kernel, p));
+    NCKV_CUDA_CHECK(cudaLaunchKernelEx(&cfg, wide ? append_rope_norm_kernel<4> : append_rope_norm_kernel<1>, p));
     return NCKV_OK;
 }
 

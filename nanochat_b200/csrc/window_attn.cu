@@ -211,6 +211,171 @@ __global__ void __launch_bounds__(256) rms_rope_append_kernel(const RmsRopeParam
           p.Hkv, p.Dv, p.Dv_pad, nullptr, 1.f, 1.f);
 }
 
+// ------------------------------------------------------------------------------------------------
+// Both appends for heads of 128 channels that are rotated as a whole, in bf16: lane j of a half-warp holds channels
+// 4j .. 4j + 3 and 64 + 4j .. 64 + 4j + 3 of a head, the two sides of its rotation pairs.
+// ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void turn4(float (&x)[4], float (&y)[4], const float (&c)[4], const float (&s)[4]) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float u = x[e], v = y[e];
+        x[e] = u * c[e] - v * s[e];
+        y[e] = v * c[e] + u * s[e];
+    }
+}
+
+// NB head rows of one token per half-warp: rows first, first + per_tok, ...
+template <int NB>
+__global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUnitParams p, int per_tok) {
+    const int j = threadIdx.x & 15, heads = p.Hq + 2 * p.Hkv;
+    const unsigned half_warp = (blockIdx.x * 256u + threadIdx.x) >> 4, n_tok = (unsigned)p.B * (unsigned)p.T;
+    unsigned tok = half_warp / (unsigned)per_tok;
+    const int first = (int)(half_warp - tok * (unsigned)per_tok);
+    bool ok = tok < n_tok;
+    if (!ok) tok = n_tok - 1;  // stays for the shuffles
+    const int b = (int)(tok / (unsigned)p.T), t = (int)(tok - (unsigned)b * (unsigned)p.T);
+    float x[NB][4], y[NB][4];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int hh = first + i * per_tok;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[i][e] = y[i][e] = 0.f;
+        if (!ok || hh >= heads) continue;
+        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + p.Hkv;
+        const int h = is_q ? hh : (is_v ? hh - p.Hq - p.Hkv : hh - p.Hq);
+        const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(is_q ? p.q : (is_v ? p.v : p.k)) +
+                                   tok * (is_q ? p.q_stride : (is_v ? p.v_stride : p.k_stride)) + h * 128 + 4 * j;
+        get_v(src, x[i]);
+        get_v(src + 64, y[i]);
+    }
+    const int L = p.seqlens[b], pos = L + t;
+    if (ok && (L < 0 || pos >= p.T_max || pos >= p.rope_len)) {
+        if (j == 0) atomicOr(p.status, (int)(L < 0 ? NCKV_ST_BAD_SEQLEN : NCKV_ST_OVERFLOW));
+        ok = false;
+    }
+    float c[4] = {0.f, 0.f, 0.f, 0.f}, s[4] = {0.f, 0.f, 0.f, 0.f};
+    if (ok) {
+        get_v(p.cs + (long long)pos * 128 + 4 * j, c);
+        get_v(p.cs + (long long)pos * 128 + 64 + 4 * j, s);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+        const int hh = first + i * per_tok;
+        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + p.Hkv;
+        const int h = is_q ? hh : (is_v ? hh - p.Hq - p.Hkv : hh - p.Hq);
+        if (__any_sync(0xffffffffu, !is_v)) {  // the other half-warp may hold another kind of row
+            float u[4], v[4], ss = 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                u[e] = x[i][e];
+                v[e] = y[i][e];
+            }
+            turn4(u, v, c, s);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ss = fmaf(u[e], u[e], fmaf(v[e], v[e], ss));
+#pragma unroll
+            for (int off = 8; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+            float f = rsqrtf(ss * (1.f / 128.f) + p.eps);
+            if (is_q) f *= p.q_scale;
+            if (!is_v) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    x[i][e] = u[e] * f;
+                    y[i][e] = v[e] * f;
+                }
+            }
+        }
+        if (!ok || hh >= heads) continue;
+        __nv_bfloat16 *dst = is_q ? static_cast<__nv_bfloat16 *>(p.q_out) + ((long long)tok * p.Hq + h) * 128
+                             : is_v ? static_cast<__nv_bfloat16 *>(p.v_cache) + b * p.vcache_bs + pos * p.vcache_ts + h * 128
+                                    : static_cast<__nv_bfloat16 *>(p.k_cache) + b * p.cache_bs + pos * p.cache_ts + h * 128;
+        put_v(dst + 4 * j, x[i]);
+        put_v(dst + 64 + 4 * j, y[i]);
+    }
+}
+
+// One CTA per token; a thread holds its NI pieces of q, k and v from the norm's sums to the store.
+template <int NI>
+__global__ void __launch_bounds__(256) rms_rope_append_128_kernel(const RmsRopeParams r) {
+    const RopeUnitParams &p = r.a;
+    __shared__ float s_part[2][8];
+    const int tid = threadIdx.x, j = tid & 15;
+    const long long row = blockIdx.x;
+    const int b = (int)(blockIdx.x / (unsigned)p.T), t = (int)(blockIdx.x - (unsigned)b * (unsigned)p.T);
+    const int Hk = p.k ? p.Hkv : 0, heads = p.Hq + 2 * Hk;
+    float x[NI][4], y[NI][4], sq = 0.f, sk = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int hh = (tid >> 4) + 16 * i;
+        if (hh >= heads) continue;
+        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + Hk;
+        const int h = is_q ? hh : (is_v ? hh - p.Hq - Hk : hh - p.Hq);
+        const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(is_q ? p.q : (is_v ? p.v : p.k)) +
+                                   row * (is_q ? p.q_stride : (is_v ? p.v_stride : p.k_stride)) + h * 128 + 4 * j;
+        get_v(src, x[i]);
+        get_v(src + 64, y[i]);
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss = fmaf(x[i][e], x[i][e], fmaf(y[i][e], y[i][e], ss));
+        if (is_q) sq += ss;
+        else if (!is_v) sk += ss;
+    }
+    const int L = p.seqlens[b], pos = L + t;
+    if (L < 0 || pos >= p.T_max || pos >= p.rope_len) {  // uniform over the CTA
+        if (tid == 0) atomicOr(p.status, (int)(L < 0 ? NCKV_ST_BAD_SEQLEN : NCKV_ST_OVERFLOW));
+        return;
+    }
+    float c[4], s[4];
+    get_v(p.cs + (long long)pos * 128 + 4 * j, c);
+    get_v(p.cs + (long long)pos * 128 + 64 + 4 * j, s);
+#pragma unroll
+    for (int off = 16; off; off >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, off);
+        sk += __shfl_xor_sync(0xffffffffu, sk, off);
+    }
+    if ((tid & 31) == 0) {
+        s_part[0][tid >> 5] = sq;
+        s_part[1][tid >> 5] = sk;
+    }
+    __syncthreads();
+    sq = sk = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        sq += s_part[0][i];
+        sk += s_part[1][i];
+    }
+    const float fq = 1.f / sqrtf(sq / (float)(p.Hq * 128) + p.eps), fk = Hk ? 1.f / sqrtf(sk / (float)(Hk * 128) + p.eps) : 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+        const int hh = (tid >> 4) + 16 * i;
+        if (hh >= heads) continue;
+        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + Hk;
+        const int h = is_q ? hh : (is_v ? hh - p.Hq - Hk : hh - p.Hq);
+        if (!is_v) {
+            float w[4], v[4];
+            const float f = is_q ? fq : fk, scale = is_q ? p.q_scale : 1.f;
+            get_v((is_q ? r.q_w : r.k_w) + h * 128 + 4 * j, w);
+            get_v((is_q ? r.q_w : r.k_w) + h * 128 + 64 + 4 * j, v);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                x[i][e] *= f * w[e];
+                y[i][e] *= f * v[e];
+            }
+            turn4(x[i], y[i], c, s);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                x[i][e] *= scale;
+                y[i][e] *= scale;
+            }
+        }
+        __nv_bfloat16 *dst = is_q ? static_cast<__nv_bfloat16 *>(p.q_out) + (row * p.Hq + h) * 128
+                             : is_v ? static_cast<__nv_bfloat16 *>(p.v_cache) + b * p.vcache_bs + pos * p.vcache_ts + h * 128
+                                    : static_cast<__nv_bfloat16 *>(p.k_cache) + b * p.cache_bs + pos * p.cache_ts + h * 128;
+        put_v(dst + 4 * j, x[i]);
+        put_v(dst + 64 + 4 * j, y[i]);
+    }
+}
+
 struct WindowAttnParams {
     const void *q, *k, *v;  // q (B, T, Hq, Dk) packed; caches with the strides below
     void *out;              // (B, T, Hq, Dv) packed
@@ -341,7 +506,15 @@ int nckv_rope_unit_append(const void *q, const void *k, const void *v, int64_t q
     if (blocks > 32LL * sm_count()) blocks = 32LL * sm_count();
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)blocks;
-    if (f32) {
+    const bool whole = Dk == 128 && Dv == 128 && Dk_pad == 128 && Dv_pad == 128 && rot_dims == 128 && ((uintptr_t)cos_sin & 15) == 0;
+    if (!f32 && vec && whole && n <= 0xfffffff0LL) {
+        const int heads = Hq + 2 * Hkv;
+        const bool wide = n >= 32768;  // the chip is full either way: four rows share a table row and the index arithmetic
+        const int per_tok = wide ? (heads + 3) / 4 : heads;
+        const unsigned ctas = (unsigned)(((long long)B * T * per_tok + 15) / 16);
+        if (wide) rope_unit_append_128_kernel<4><<<ctas, 256, 0, s>>>(p, per_tok);
+        else rope_unit_append_128_kernel<1><<<ctas, 256, 0, s>>>(p, per_tok);
+    } else if (f32) {
         if (vec) rope_unit_append_kernel<float, 4><<<grid, 256, 0, s>>>(p);
         else rope_unit_append_kernel<float, 1><<<grid, 256, 0, s>>>(p);
     } else {
@@ -389,7 +562,14 @@ int nckv_rms_rope_append(const void *q, const void *k, const void *v, int64_t q_
     const bool vec = (a & (4 * elem - 1)) == 0 && (((uintptr_t)q_weight | (uintptr_t)k_weight) & 15) == 0 && rot_dims % 8 == 0;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)(B * T);
-    if (f32) {
+    const int pieces = (Hq + (k ? 2 * Hkv : 0) + 15) / 16;  // of a thread, 16 heads at a time
+    const bool whole = Dk == 128 && Dv == 128 && Dk_pad == 128 && Dv_pad == 128 && rot_dims == 128 && ((uintptr_t)cos_sin & 15) == 0;
+    if (!f32 && vec && whole && pieces <= 4) {
+        if (pieces == 1) rms_rope_append_128_kernel<1><<<grid, 256, 0, s>>>(r);
+        else if (pieces == 2) rms_rope_append_128_kernel<2><<<grid, 256, 0, s>>>(r);
+        else if (pieces == 3) rms_rope_append_128_kernel<3><<<grid, 256, 0, s>>>(r);
+        else rms_rope_append_128_kernel<4><<<grid, 256, 0, s>>>(r);
+    } else if (f32) {
         if (vec) rms_rope_append_kernel<float, 4><<<grid, 256, 0, s>>>(r);
         else rms_rope_append_kernel<float, 1><<<grid, 256, 0, s>>>(r);
     } else {
