@@ -383,11 +383,14 @@ NCKV_API int nckv_flash_attn_bwd(const void *q, const void *k, const void *v, co
  * nckv_glue_ve_gate: v_out = bf16(v + bf16(bf16(3 * bf16(sigmoid(gate_lin))) * ve)) with v, ve (rows, Hkv, D)
  * and gate_lin (rows, Hkv) the output of the gate's linear layer: the value residual of gpt.py:92-95.  v may have
  * its own row stride in elements (v_row_stride, 0 = packed): a column slice of a projection output.
+ * nckv_glue_logit_cap: out = cap * tanh(float(z) * (1 / cap)), z bf16 rows of `cols` with their own row stride, out
+ * packed fp32: the soft cap on the logits (gpt.py:469-472).
  */
 NCKV_API int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
                        void *out_x, void *out_norm, int rows, int C, int mode, float resid_lambda, float x0_lambda,
                        float backout_lambda, float eps, void *stream);
 NCKV_API int nckv_glue_relu_sq(const void *h, void *out, int64_t n, void *stream);
+NCKV_API int nckv_glue_logit_cap(const void *z, int64_t z_row_stride, float *out, int64_t rows, int cols, float cap, void *stream);
 NCKV_API int nckv_glue_ve_gate(const void *v, int64_t v_row_stride, const void *gate_lin, const void *ve, void *v_out, int rows, int Hkv, int D,
                       void *stream);
 

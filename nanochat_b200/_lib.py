@@ -46,6 +46,7 @@ SIGNATURES = {
                                       ctypes.c_uint64, c_void_p]),
     "nckv_glue_mix_norm": (c_int, [c_void_p] * 7 + [c_int] * 3 + [c_float] * 4 + [c_void_p]),
     "nckv_glue_relu_sq": (c_int, [c_void_p, c_void_p, c_i64, c_void_p]),
+    "nckv_glue_logit_cap": (c_int, [c_void_p, c_i64, c_void_p, c_i64, c_int, c_float, c_void_p]),
     "nckv_glue_ve_gate": (c_int, [c_void_p, c_i64] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p]),
     "nckv_append_rope_norm_strided": (c_int, [c_void_p] * 3 + [c_i64] * 3 + [c_void_p] * 6 + [c_int] * 6 + [c_i64, c_i64, c_int, c_float, c_float,
                                               c_void_p, c_void_p]),

@@ -1,4 +1,4 @@
-// Decode-time elementwise glue of the transformer trunk, fused per layer and bit-exact against the
+// Elementwise glue of the transformer trunk, fused per layer and bit-exact against the
 // eager bf16 op sequence it replaces (every eager op computes in fp32 and rounds its result to bf16;
 // the kernels round at the same points).
 //
@@ -12,9 +12,13 @@
 //                     block of 32 x 4 threads, thread t accumulates the 4-element vectors t, t + 128,
 //                     ... sequentially (fused multiply-add), then a shuffle-down tree inside each warp
 //                     (offsets 16, 8, 4, 2, 1), then warps (0 += 2, 1 += 3), then 0 += 1.
+//                     A row's operands are all loaded before anything is stored (NV vectors per thread,
+//                     a template constant): stores that might alias kept each vector's loads behind the one before.
 //   relu_sq_kernel    bf16(max(h, 0)^2)                                               MLP            (gpt.py:136)
 //   ve_gate_kernel    bf16(v + bf16(bf16(3 * bf16(sigmoid(g))) * ve))                 value residual (gpt.py:92-95)
-#include "nckv_common.cuh"
+//   logit_cap_kernel  cap * tanh(float(z) * (1 / cap)), bf16 in, fp32 out               logits         (gpt.py:469-472)
+//                     One pass over the logits (6 bytes each) where the eager ops take four (30 bytes each).
+#include "vec_io.cuh"
 
 namespace nckv {
 
@@ -39,37 +43,47 @@ __device__ __forceinline__ uint2 pack4(const float (&f)[4]) {
     return v;
 }
 
+// NV: vectors of 4 channels per thread
+template <int NV>
 __global__ void __launch_bounds__(GLUE_THREADS) glue_row_kernel(const GlueRowParams p) {
     __shared__ float s_buf[4];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int n_vec = p.C >> 2;
     const long long base = (long long)blockIdx.x * n_vec;
-    float y[GLUE_MAX_VEC][4];
+    const uint2 *second = p.mode == 1 ? p.x0 : p.xb;
+    uint2 in[NV], in_add[NV], in_second[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = t + k * GLUE_THREADS;
+        in[k] = in_add[k] = in_second[k] = make_uint2(0, 0);
+        if (i < n_vec) {
+            in[k] = p.x[base + i];
+            if (p.add) in_add[k] = p.add[base + i];
+            if (p.mode != 0) in_second[k] = second[base + i];
+        }
+    }
+    float y[NV][4];
     float acc = 0.f;
 #pragma unroll
-    for (int k = 0; k < GLUE_MAX_VEC; ++k) {
+    for (int k = 0; k < NV; ++k) {
         const int i = t + k * GLUE_THREADS;
         if (i < n_vec) {
             float a[4];
-            unpack4(p.x[base + i], a);
+            unpack4(in[k], a);
             if (p.add) {
                 float b[4];
-                unpack4(p.add[base + i], b);
+                unpack4(in_add[k], b);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) a[e] = round_bf16(__fadd_rn(a[e], b[e]));
                 if (p.out_sum) p.out_sum[base + i] = pack4(a);
             }
-            if (p.mode == 1) {
+            if (p.mode != 0) {
                 float z[4];
-                unpack4(p.x0[base + i], z);
+                unpack4(in_second[k], z);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    a[e] = round_bf16(__fadd_rn(round_bf16(__fmul_rn(p.rl, a[e])), round_bf16(__fmul_rn(p.xl, z[e]))));
-            } else if (p.mode == 2) {
-                float z[4];
-                unpack4(p.xb[base + i], z);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) a[e] = round_bf16(__fsub_rn(a[e], round_bf16(__fmul_rn(p.bl, z[e]))));
+                    a[e] = p.mode == 1 ? round_bf16(__fadd_rn(round_bf16(__fmul_rn(p.rl, a[e])), round_bf16(__fmul_rn(p.xl, z[e]))))
+                                       : round_bf16(__fsub_rn(a[e], round_bf16(__fmul_rn(p.bl, z[e]))));
             }
             if (p.out_x) p.out_x[base + i] = pack4(a);
 #pragma unroll
@@ -92,7 +106,7 @@ __global__ void __launch_bounds__(GLUE_THREADS) glue_row_kernel(const GlueRowPar
     __syncthreads();
     const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(s_buf[1], (float)p.C), p.eps));
 #pragma unroll
-    for (int k = 0; k < GLUE_MAX_VEC; ++k) {
+    for (int k = 0; k < NV; ++k) {
         const int i = t + k * GLUE_THREADS;
         if (i < n_vec) {
             float o[4];
@@ -144,9 +158,44 @@ __global__ void __launch_bounds__(256) ve_gate_kernel(const uint4 *__restrict__ 
     }
 }
 
+// V elements at a time; rows of `cols` in an input of row stride `in_stride`
+template <int V>
+__global__ void __launch_bounds__(256) logit_cap_kernel(const __nv_bfloat16 *__restrict__ z, long long in_stride, float *__restrict__ out,
+                                                        long long rows, int cols, float inv_cap, float cap) {
+    const int per = cols / V;
+    for (long long row = blockIdx.y; row < rows; row += gridDim.y) {
+        const __nv_bfloat16 *src = z + row * in_stride;
+        float *dst = out + row * cols;
+        for (int i = blockIdx.x * 256 + threadIdx.x; i < per; i += gridDim.x * 256) {
+            float v[V];
+            get_v(src + (long long)i * V, v);
+#pragma unroll
+            for (int e = 0; e < V; ++e) v[e] = __fmul_rn(cap, tanhf(__fmul_rn(v[e], inv_cap)));
+            put_v(dst + (long long)i * V, v);
+        }
+    }
+}
+
 }  // namespace nckv
 
 extern "C" {
+
+int nckv_glue_logit_cap(const void *z, int64_t z_row_stride, float *out, int64_t rows, int cols, float cap, void *stream) {
+    using namespace nckv;
+    if (!z || !out || rows <= 0 || cols <= 0 || z_row_stride < cols || !(cap > 0.f)) {
+        set_error("glue_logit_cap: null pointer or bad size (rows=%lld cols=%d stride=%lld)", (long long)rows, cols, (long long)z_row_stride);
+        return NCKV_E_ARG;
+    }
+    const bool vec = cols % 8 == 0 && z_row_stride % 8 == 0 && (((uintptr_t)z | (uintptr_t)out) & 15) == 0;
+    const int per = vec ? cols / 8 : cols;
+    const dim3 grid((unsigned)((per + 255) / 256), (unsigned)(rows < 65535 ? rows : 65535));
+    const __nv_bfloat16 *in = static_cast<const __nv_bfloat16 *>(z);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (vec) logit_cap_kernel<8><<<grid, 256, 0, s>>>(in, z_row_stride, out, rows, cols, 1.f / cap, cap);
+    else logit_cap_kernel<1><<<grid, 256, 0, s>>>(in, z_row_stride, out, rows, cols, 1.f / cap, cap);
+    NCKV_CUDA_CHECK(cudaGetLastError());
+    return NCKV_OK;
+}
 
 int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
                        void *out_x, void *out_norm, int rows, int C, int mode, float resid_lambda, float x0_lambda,
@@ -180,7 +229,10 @@ int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const voi
     p.out_norm = static_cast<uint2 *>(out_norm);
     p.rl = resid_lambda; p.xl = x0_lambda; p.bl = backout_lambda; p.eps = eps;
     p.C = C; p.mode = mode;
-    glue_row_kernel<<<rows, GLUE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
+    const int nv = (C / 4 + GLUE_THREADS - 1) / GLUE_THREADS;
+    const auto kernel = nv == 1 ? glue_row_kernel<1> : nv == 2 ? glue_row_kernel<2> : nv == 3 ? glue_row_kernel<3> : nv == 4 ? glue_row_kernel<4>
+                        : nv <= 8 ? glue_row_kernel<8> : glue_row_kernel<GLUE_MAX_VEC>;
+    kernel<<<rows, GLUE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
     NCKV_CUDA_CHECK(cudaGetLastError());
     return NCKV_OK;
 }

@@ -213,6 +213,8 @@ class Block(nn.Module):
 class GPT(nn.Module):
     """Inference-only GPT with the reference's module tree and forward arithmetic (gpt.py:154-481)."""
 
+    accepts_logits_at = True
+
     def __init__(self, config, pad_vocab_size_to=64, compute_dtype=None):
         super().__init__()
         self.config = config
@@ -233,7 +235,7 @@ class GPT(nn.Module):
         kv_dim = config.n_kv_head * head_dim
         self.value_embeds = nn.ModuleDict({str(i): nn.Embedding(padded, kv_dim) for i in range(config.n_layer)
                                            if layer_has_value_embedding(i, config.n_layer)})
-        # Decode steps (one new token per row, CUDA, bf16) run the elementwise glue between the matrix
+        # Forward passes over a cache (CUDA, bf16) run the elementwise glue between the matrix
         # products through the fused kernels of libnckv (bit-identical to the eager ops); set False to
         # run the eager op sequence everywhere.
         self.fused_glue = True
@@ -306,9 +308,9 @@ class GPT(nn.Module):
                 ve.to(dtype=dtype)
 
     @torch.inference_mode()
-    def forward(self, idx, targets=None, kv_cache=None, loss_reduction="mean"):
-        """Logits (B, T, vocab) in fp32.  Same arithmetic as gpt.py:416-472; ``targets`` is rejected
-        (no training here)."""
+    def forward(self, idx, targets=None, kv_cache=None, loss_reduction="mean", logits_at=None):
+        """Logits (B, T, vocab) in fp32, or (B, len(logits_at), vocab) at the given places of the T tokens.
+        Same arithmetic as gpt.py:416-472; ``targets`` is rejected (no training here)."""
         if targets is not None:
             raise NotImplementedError("this GPT is inference-only")
         B, T = idx.shape
@@ -334,8 +336,9 @@ class GPT(nn.Module):
         backout_at = self.config.n_layer // 2
         x_backout = None
         rope_tables = (self.cos, self.sin)
-        if self.fused_glue and T == 1 and kv_cache is not None and x.is_cuda and x.dtype == torch.bfloat16:
-            return self._decode_trunk_fused(idx, x, kv_cache, rope_tables)
+        if self.fused_glue and kv_cache is not None and x.is_cuda and x.dtype == torch.bfloat16 and \
+                (T == 1 or self._prompt_can_fuse(B)):
+            return self._head(self._trunk_fused(idx, x, kv_cache, rope_tables), logits_at)
         for i, block in enumerate(self.transformer.h):
             x = self.resid_lambdas[i] * x + self.x0_lambdas[i] * x0
             ve = self.value_embeds[str(i)](idx).to(x.dtype) if str(i) in self.value_embeds else None
@@ -344,28 +347,46 @@ class GPT(nn.Module):
                 x_backout = x
         if x_backout is not None:
             x = x - self.backout_lambda.to(x.dtype) * x_backout
-        x = rms(x)
-        logits = self.lm_head(x)[..., :self.config.vocab_size].float()
-        return 15 * torch.tanh(logits / 15)
+        return self._head(rms(x), logits_at)
+
+    def _prompt_can_fuse(self, rows):
+        """The fused trunk reads the lambdas on the host once per version, which a stream capture does not allow and
+        inference tensors do not have, and it has a widest row; the eager trunk takes the rest."""
+        if rows == 0 or self.config.n_embd > ops.GLUE_MAX_C or self.resid_lambdas.is_inference():
+            return False
+        known = self._lambda_cache is not None and self._lambda_cache[0] == self._lambda_key()
+        return known or not torch.cuda.is_current_stream_capturing()
+
+    def _head(self, x, logits_at):
+        """Soft-capped logits of normed activations (B, T, C), at the given places only if there are any given."""
+        if logits_at is not None:
+            x = x[:, logits_at]
+        z = self.lm_head(x)
+        if self.fused_glue and z.is_cuda and z.dtype == torch.bfloat16:
+            return ops.glue_logit_cap(z, self.config.vocab_size, 15.0)
+        return 15 * torch.tanh(z[..., :self.config.vocab_size].float() / 15)
+
+    def _lambda_key(self):
+        return (self.resid_lambdas.data_ptr(), self.resid_lambdas._version, self.x0_lambdas._version,
+                self.backout_lambda._version, self.resid_lambdas.dtype)
 
     def _lambdas(self):
         """Host copies of the per-layer scalars, read once (a device read per step would synchronise),
         rounded to bf16: the eager multiply converts a 0-dim parameter to the activation dtype before it
         multiplies (and gpt.py:467 casts the backout lambda explicitly)."""
-        key = (self.resid_lambdas.data_ptr(), self.resid_lambdas._version, self.x0_lambdas._version,
-               self.backout_lambda._version, self.resid_lambdas.dtype)
+        key = self._lambda_key()
         if self._lambda_cache is None or self._lambda_cache[0] != key:
             as_bf16 = lambda t: t.detach().to(torch.bfloat16).float()
             self._lambda_cache = (key, as_bf16(self.resid_lambdas).tolist(), as_bf16(self.x0_lambdas).tolist(),
                                   float(as_bf16(self.backout_lambda).item()))
         return self._lambda_cache[1:]
 
-    def _decode_trunk_fused(self, idx, x, kv_cache, rope_tables):
-        """The layer loop of ``forward`` for one new token per row with the elementwise glue fused:
+    def _trunk_fused(self, idx, x, kv_cache, rope_tables):
+        """The layer loop of ``forward`` over a cache with the elementwise glue fused, up to the last norm:
         per layer one launch for [previous MLP residual add + lambda mix + norm], one for [attention
         residual add + norm], one for relu^2 (and one for the value-embedding gate where a layer has
         one), instead of about a dozen eager launches.  Same matrix products, same roundings."""
-        B = idx.size(0)
+        B, T = idx.shape
         C = x.size(-1)
         resid, x0l, backout = self._lambdas()
         n_layer = self.config.n_layer
@@ -381,7 +402,8 @@ class GPT(nn.Module):
             if i == backout_at + 1:
                 x_backout = x_sum
             attn = block.attn
-            w_qkv = attn.fused_qkv_weight(xn) if self.fused_qkv else None
+            # one token per row: the row count stays, and with it the check; prompts come in all lengths
+            w_qkv = attn.fused_qkv_weight(xn) if self.fused_qkv and T == 1 else None
             if w_qkv is not None:  # one product; q, k, v are column slices of its output (the kernels take the stride)
                 nq, nkv = attn.n_head * attn.head_dim, attn.n_kv_head * attn.head_dim
                 qkv = F.linear(xn, w_qkv)
@@ -389,22 +411,21 @@ class GPT(nn.Module):
                 k = qkv[..., nq:nq + nkv].view(B, 1, attn.n_kv_head, attn.head_dim)
                 v = qkv[..., nq + nkv:].view(B, 1, attn.n_kv_head, attn.head_dim)
             else:
-                q = attn.c_q(xn).view(B, 1, attn.n_head, attn.head_dim)
-                k = attn.c_k(xn).view(B, 1, attn.n_kv_head, attn.head_dim)
-                v = attn.c_v(xn).view(B, 1, attn.n_kv_head, attn.head_dim)
+                q = attn.c_q(xn).view(B, T, attn.n_head, attn.head_dim)
+                k = attn.c_k(xn).view(B, T, attn.n_kv_head, attn.head_dim)
+                v = attn.c_v(xn).view(B, T, attn.n_kv_head, attn.head_dim)
             if str(i) in self.value_embeds:
                 ve = self.value_embeds[str(i)](idx).to(x.dtype)
                 v = ops.glue_ve_gate(v, attn.ve_gate(xn[..., :attn.ve_gate_channels]), ve)
             y = kv_attention(q, k, v, rope_tables, self.window_sizes[i], kv_cache, i)
-            _, x, xn = ops.glue_mix_norm(x, add=attn.c_proj(y.view(B, 1, C)))
+            _, x, xn = ops.glue_mix_norm(x, add=attn.c_proj(y.view(B, T, C)))
             pending = block.mlp.c_proj(ops.glue_relu_sq(block.mlp.c_fc(xn)))
         if backout_at == n_layer - 1:  # only a one-layer model: the backout operand is the final sum itself
             x_backout, _, _ = ops.glue_mix_norm(x, add=pending, want_sum=True, want_x=False, want_norm=False)
             _, _, xn = ops.glue_mix_norm(x_backout, x_backout=x_backout, backout_lambda=backout, want_x=False)
         else:
             _, _, xn = ops.glue_mix_norm(x, add=pending, x_backout=x_backout, backout_lambda=backout, want_x=False)
-        logits = self.lm_head(xn)[..., :self.config.vocab_size].float()
-        return 15 * torch.tanh(logits / 15)
+        return xn
 
     @torch.inference_mode()
     def generate(self, tokens, max_tokens, temperature=1.0, top_k=None, seed=42):

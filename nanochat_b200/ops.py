@@ -714,6 +714,23 @@ def glue_relu_sq(h):
     return out
 
 
+def glue_logit_cap(z, cols, cap):
+    """cap * tanh(z / cap) of the first ``cols`` channels of bf16 rows, in fp32 and one launch (gpt.py:469-472)."""
+    if not z.is_cuda or z.dtype != torch.bfloat16 or not z.is_contiguous() or z.size(-1) < cols:
+        raise RuntimeError(f"nckv::glue_logit_cap needs contiguous CUDA bfloat16 rows of at least {cols} channels")
+    out = torch.empty(*z.shape[:-1], cols, dtype=torch.float32, device=z.device)
+    rows = z.numel() // z.size(-1)
+    if rows:
+        idx = z.device.index
+        with _device_guard(idx):
+            _lib.call("nckv_glue_logit_cap", z.data_ptr(), z.size(-1), out.data_ptr(), rows, cols, float(cap),
+                      torch.cuda.current_stream(idx).cuda_stream)
+    return out
+
+
+GLUE_MAX_C = 8192  # widest rows of glue_mix_norm
+
+
 def glue_ve_gate(v, gate_lin, ve):
     """v + 3 * sigmoid(gate_lin)[..., None] * ve in one launch (gpt.py:92-95); v, ve: (..., Hkv, 128),
     gate_lin: (..., Hkv) — the output of the gate's linear layer."""
