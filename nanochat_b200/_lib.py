@@ -125,6 +125,12 @@ def _load():
 
 
 lib = _load()
+try:
+    import torch  # noqa: F401  (its libraries first: _native is linked against them)
+
+    from . import _native as native  # the most repeated calls without ctypes; None from one of them: take the general path
+except ImportError as e:
+    raise ImportError(f"nanochat_b200/_native.so cannot be loaded ({e}): build it with `python -m nanochat_b200.csrc.build`") from e
 
 
 def check(fn_name, rc):

@@ -1,19 +1,22 @@
-"""Build libnckv.so (all CUDA sources of this directory) for sm_100a with nvcc.
+"""Build libnckv.so (all CUDA sources of this directory) for sm_100a with nvcc, and _native.so (binding.cpp: the most
+repeated calls from torch tensors to the library) with the host compiler.
 
 Usage:  python -m nanochat_b200.csrc.build [--verbose] [--force]
-The shared library is written next to the package (nanochat_b200/libnckv.so); it is a build
-artefact and is not tracked.
+Both are written next to the package (nanochat_b200/); they are build artefacts and are not tracked.
 """
 import fcntl
 import os
 import subprocess
 import sys
+import sysconfig
 import tempfile
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 OUT = os.path.join(PKG, "libnckv.so")
+NATIVE = os.path.join(PKG, "_native.so")
+BINDING = os.path.join(HERE, "binding.cpp")
 SOURCES = ["host.cu", "append.cu", "decode_attn.cu", "prefill_broadcast.cu", "lse_combine.cu",
            "prefill_attn.cu", "p2p_exchange.cu", "glue.cu", "flash_attn_bwd.cu", "host_step.cu",
            "recurrent.cu", "recurrent_f32.cu", "norm_mix.cu", "window_attn.cu", "hyper_norm.cu",
@@ -29,11 +32,27 @@ def _nvcc():
 
 
 def up_to_date():
-    if not os.path.exists(OUT):
+    return _newer(OUT, [os.path.join(HERE, s) for s in SOURCES + HEADERS]) and _newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])])
+
+
+def _newer(built, deps):
+    if not os.path.exists(built):
         return False
-    t = os.path.getmtime(OUT)
-    deps = [os.path.join(HERE, s) for s in SOURCES + HEADERS] + [os.path.abspath(__file__)]
-    return all(os.path.getmtime(d) <= t for d in deps)
+    t = os.path.getmtime(built)
+    return all(os.path.getmtime(d) <= t for d in deps + [os.path.abspath(__file__)])
+
+
+def _binding_command(out):
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    include = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+               os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    libs = ["c10", "c10_cuda", "torch", "torch_cpu", "torch_cuda", "torch_python"]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_native",
+            *[f"-I{d}" for d in include], BINDING, "-o", out, f"-L{os.path.join(base, 'lib')}", *[f"-l{n}" for n in libs],
+            f"-L{PKG}", "-l:libnckv.so", "-Wl,-rpath,$ORIGIN"]
 
 
 def _compile(cmd, verbose):
@@ -44,7 +63,7 @@ def _compile(cmd, verbose):
 
 
 def build(verbose=False, force=False):
-    """Compile the sources side by side, link them, and move the library into place in one step; several
+    """Compile the sources side by side, link them, and move each library into place in one step; several
     processes may call this at the same time."""
     if not force and up_to_date():
         return OUT
@@ -55,15 +74,17 @@ def build(verbose=False, force=False):
         nvcc = _nvcc()
         flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
                  "-Xcompiler", "-fvisibility=hidden"] + (["-Xptxas", "-v"] if verbose else [])
-        with tempfile.TemporaryDirectory(dir=PKG, prefix=".build-") as tmp:
+        with tempfile.TemporaryDirectory(dir=PKG, prefix=".build-") as tmp, ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
             objs = [os.path.join(tmp, os.path.splitext(s)[0] + ".o") for s in SOURCES]
             jobs = [[nvcc] + flags + ["-c", "-o", o, os.path.join(HERE, s)] for s, o in zip(SOURCES, objs)]
-            with ThreadPoolExecutor(max(1, min(len(jobs), os.cpu_count() or 1))) as pool:
-                failed = any(list(pool.map(lambda cmd: _compile(cmd, verbose), jobs)))
-            linked = os.path.join(tmp, os.path.basename(OUT))
-            if failed or _compile([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "--shared", "-o", linked] + objs, verbose):
+            linked, native = os.path.join(tmp, os.path.basename(OUT)), os.path.join(tmp, os.path.basename(NATIVE))
+            if any(list(pool.map(lambda cmd: _compile(cmd, verbose), jobs))) or \
+                    _compile([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "--shared", "-o", linked] + objs, verbose):
                 raise RuntimeError("nvcc failed building libnckv.so")
             os.replace(linked, OUT)
+            if _compile(_binding_command(native), verbose):
+                raise RuntimeError("the host compiler failed building _native.so")
+            os.replace(native, NATIVE)
     return OUT
 
 

@@ -213,7 +213,9 @@ __global__ void __launch_bounds__(256) rms_rope_append_kernel(const RmsRopeParam
 
 // ------------------------------------------------------------------------------------------------
 // Both appends for heads of 128 channels that are rotated as a whole, in bf16: lane j of a half-warp holds channels
-// 4j .. 4j + 3 and 64 + 4j .. 64 + 4j + 3 of a head, the two sides of its rotation pairs.
+// 4j .. 4j + 3 and 64 + 4j .. 64 + 4j + 3 of a head, the two sides of its rotation pairs.  The general kernels load
+// every pair twice, table entries one by one, and divide 64-bit indices per head row: 183 us against 88 us for
+// 8 x 2048 tokens of 36 heads (rope_unit), 47 us against 41 us for 6007 tokens of 36 heads (rms_rope).
 // ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void turn4(float (&x)[4], float (&y)[4], const float (&c)[4], const float (&s)[4]) {
 #pragma unroll

@@ -66,7 +66,13 @@ def kv_attention(q, k, v, cos_sin_tables, window_size, kv_cache, layer_idx):
     T = q.size(1)
     left = int(window_size[0])
     left = left if left >= 0 else -1
-    if getattr(kv_cache, "paged", False):  # page pools + block table instead of dense rows
+    paged = getattr(kv_cache, "paged", False)
+    y = ops.append_and_attend(q, k, v, k_cache, v_cache, kv_cache.block_table if paged else None, seqlens, cos, sin, left)
+    if y is not None:
+        if layer_idx == kv_cache.n_layers - 1:
+            kv_cache.advance(T)
+        return y
+    if paged:  # page pools + block table instead of dense rows
         if T != 1:
             raise NotImplementedError("a paged cache takes one new token per row; prefill the prompt into a dense "
                                       "batch-1 KVCache and hand it over with PagedKVCache.prefill")

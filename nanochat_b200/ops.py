@@ -113,6 +113,7 @@ def workspace(device, B, Hq, Hkv):
             _retired_workspaces.append(ws)
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=torch.device("cuda", idx))
         _workspaces[key] = ws
+        _lib.native.set_workspace(*key, ws)
     return ws
 
 
@@ -483,6 +484,12 @@ def append_rope_norm(q, k, v, k_cache, v_cache, cache_seqlens, cos, sin, qk_scal
     return _append_rope_norm(q, k, v, k_cache, v_cache, cache_seqlens, cos, sin, qk_scale, eps, write_slots, split)
 
 
+def append_and_attend(q, k, v, k_cache, v_cache, block_table, cache_seqlens, cos, sin, window_left):
+    """``append_rope_norm`` and the attention behind it (one or several new tokens per row, dense rows or, with a
+    ``block_table``, page pools) as one native call; returns (B, T, Hq, D), or None where only the single calls apply."""
+    return _lib.native.kv_attention(q, k, v, k_cache, v_cache, block_table, cache_seqlens, cos, sin, window_left, QK_SCALE, RMS_EPS)
+
+
 def decode_attention_split(q, k_cache, v_cache, cache_seqlens, split, part_out, part_lse, seqlen_offset=1,
                            peer_ptrs=None, step_counter=None):
     """One-token attention over this rank's block-cyclic part of the keys (``split = (world, rank,
@@ -686,6 +693,9 @@ def glue_mix_norm(x, add=None, x0=None, x_backout=None, resid_lambda=1.0, x0_lam
     ``a - backout_lambda * x_backout`` (when ``x_backout`` is given); then rms-norm.  Every step
     rounds to bf16 like the eager op it stands for.  Returns (a or None, y or None, norm or None)."""
     name = "glue_mix_norm"
+    done = _lib.native.glue_mix_norm(x, add, x0, x_backout, resid_lambda, x0_lambda, backout_lambda, want_sum, want_x, want_norm, eps)
+    if done is not None:
+        return done
     C = x.size(-1)
     px = _rows(name, x, C)
     rows = x.numel() // C
@@ -705,6 +715,9 @@ def glue_mix_norm(x, add=None, x0=None, x_backout=None, resid_lambda=1.0, x0_lam
 
 def glue_relu_sq(h):
     """relu(h)^2 in one launch (MLP.forward, gpt.py:136), bf16 rounding after each of the two eager ops."""
+    done = _lib.native.glue_relu_sq(h)
+    if done is not None:
+        return done
     if not h.is_cuda or h.dtype != torch.bfloat16 or not h.is_contiguous():
         raise RuntimeError("nckv::glue_relu_sq needs a contiguous CUDA bfloat16 tensor")
     out = torch.empty_like(h)
