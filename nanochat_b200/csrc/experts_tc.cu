@@ -152,7 +152,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         }
     } else if (warp == 1) {
         // =============== products ===================================================================
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t IDESC = umma_idesc(ET_M, BN, 0, 0);
             const uint64_t desc0 = smem_desc_sw128(smem_u32(smem), 16, 1024);
             uint32_t fill = 0, tile = 0;

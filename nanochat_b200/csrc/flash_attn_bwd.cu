@@ -217,7 +217,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
     if (warp == BT_EW_THREADS / 32 + 1) {
         // =============== one thread issues the copies ================================================
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(&sh.bar_own, 2 * BT_TILE_BYTES);
             bt_load_tile(sK, &tmap_k, &sh.bar_own, hkv, k0, b);
             bt_load_tile(sV, &tmap_v, &sh.bar_own, hkv, k0, b);
@@ -243,7 +243,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         __syncwarp();
     } else if (warp == BT_EW_THREADS / 32) {
         // =============== one thread issues the products ==============================================
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             const uint64_t desc_k = smem_desc_sw128(smem_u32(sK), 16, 1024);
             const uint64_t desc_v = smem_desc_sw128(smem_u32(sV), 16, 1024);
             const uint32_t ring_addr = smem_u32(ring);
@@ -471,7 +471,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
     if (warp == BT_EW_THREADS / 32 + 1) {
         // =============== one thread issues the copies ================================================
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(&sh.bar_own, 2 * BT_TILE_BYTES);
             bt_load_tile(sQ, &tmap_q, &sh.bar_own, hq, q0, b);
             bt_load_tile(sdO, &tmap_do, &sh.bar_own, hq, q0, b);
@@ -496,7 +496,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         __syncwarp();
     } else if (warp == BT_EW_THREADS / 32) {
         // =============== one thread issues the products ==============================================
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             const uint64_t desc_q = smem_desc_sw128(smem_u32(sQ), 16, 1024);
             const uint64_t desc_do = smem_desc_sw128(smem_u32(sdO), 16, 1024);
             const uint32_t ring_addr = smem_u32(ring);

@@ -222,7 +222,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 
     if (warp == PF_SOFTMAX_THREADS / 32 + 1) {
         // =============== one lane moves the tiles ===================================================
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             PfCursor kc, vc, wc;  // next K tile to load, next V tile to load, tile whose score product is awaited
             kc.load(p, 0);
             vc = kc;
@@ -278,7 +278,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         // =============== one thread feeds the tensor core ==========================================
         // tcgen05.mma / tcgen05.commit are single-thread instructions and an mbarrier poll by 32 lanes
         // is 32 polls, one after the other: lane 0 runs this role alone.
-        if ((tid & 31) == 0) {
+        if (elect_one()) {
             // Descriptors differ only in the start-address field (address >> 4 in the low 14 bits),
             // so they are built once and advanced by adding the byte offset >> 4.
             const uint64_t desc_q = smem_desc_sw128(smem_u32(sQ), 16, 1024);
