@@ -7,11 +7,15 @@
 //   warp 0      moves the weights, and without UP the positions (rows of act), by TMA
 //   warps 6-13  UP: the tokens of a tile lie anywhere in h; these warps fetch them with 16-byte asynchronous copies
 //               into the place the swizzle gives them, so h is never copied into sorted order (a gather by
-//               TMA, four rows per instruction, was three times slower than the products).  Four of the
-//               warps take the even steps, four the odd ones.
+//               TMA, four rows per instruction, was three times slower than the products).  With four stages four
+//               groups of two warps take a step each in turn; a group waits for its own copies, so four steps
+//               are on their way at any time (two groups that handed a step over behind the next one's request
+//               had two: 178 us at 6007 tokens x 4 of 16 experts of 1536 x 1024, now 154).
 //   warp 1      one thread issues the products into one of two accumulators
 //   warps 2-5   one thread per position reads the other accumulator, applies the router's weight and the
-//               activation (UP) or finds the pair's place (down), and stores
+//               activation (UP) or finds the pair's place (down); results are turned in shared memory and stored 128
+//               bytes of a row by 8 lanes (16 bytes of 32 rows per instruction held up the operands of the next
+//               tile's products: down 83 us, now 69)
 // Tiles of one expert are consecutive, positions fastest: the CTAs that run side by side share weights and rows
 // in L2.  What stands in a tile behind an expert's last position is not stored.  Every wait is bounded; one that
 // runs out sets NCKV_ST_TIMEOUT, the roles stop, copies in flight are waited for and tensor memory is freed.
@@ -22,13 +26,15 @@ namespace nckv {
 
 constexpr int ET_M = 128, ET_K = 64;
 constexpr int ET_THREADS = 192, ET_GATHER = 256;  // UP has ET_GATHER more, in two halves
+template <int STAGES> constexpr int ET_GROUPS = STAGES == 4 ? 4 : 2;  // groups of warps that fetch tokens: a divisor of the stages
 constexpr int ET_MAX_EXPERTS = 1024;
 constexpr int ET_A_BYTES = ET_M * ET_K * 2;
+constexpr int ET_OUT_BYTES = 4 * 32 * 128;  // a warp's 32 rows by 64 results on their way out
 
 template <int BN> struct EtShape {
     static constexpr int B_BYTES = BN * ET_K * 2, STAGE = ET_A_BYTES + B_BYTES;
     static constexpr int STAGES = BN == 256 ? 4 : 6;
-    static constexpr int SMEM = STAGES * STAGE + 256;
+    static constexpr int SMEM = STAGES * STAGE + ET_OUT_BYTES + 256;
 };
 
 // One tile, found by walking on from the tile before.
@@ -57,7 +63,8 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (threadIdx.x == 0) atomicOr(p.status, (int)NCKV_ST_TIMEOUT);
         return;
     }
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + STAGES * Shape::STAGE);
+    uint8_t *s_out = smem + STAGES * Shape::STAGE;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(s_out + ET_OUT_BYTES);
     uint64_t *bar_full = bars, *bar_free = bars + STAGES;                         // a stage's operands landed / were read
     uint64_t *bar_acc = bars + 2 * STAGES, *bar_read = bars + 2 * STAGES + 2;     // an accumulator is complete / was read
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + 4);
@@ -87,7 +94,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         prefetch_tensormap(&map_a);
         prefetch_tensormap(&map_w);
         for (int i = 0; i < STAGES; ++i) {
-            mbar_init(&bar_full[i], UP ? 1 + ET_GATHER / 64 : 1);
+            mbar_init(&bar_full[i], UP ? 1 + ET_GATHER / 32 / ET_GROUPS<STAGES> : 1);
             mbar_init(&bar_free[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -118,18 +125,19 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     cur.e = 0;
     if (warp == 0) {
         // =============== operands ===================================================================
-        uint32_t fill = 0;  // number of the fill: stage fill % STAGES
-        bool ok = true;
-        for (int idx = blockIdx.x; idx < total && ok; idx += gridDim.x) {
-            if (!cur.seek(s_first, p, n_tiles, idx)) break;
-            for (int ks = 0; ks < k_steps; ++ks, ++fill) {
-                const uint32_t st = fill % STAGES, round = fill / STAGES;
-                if (round > 0 && !warp_wait(&bar_free[st], (round - 1) & 1u)) {
-                    ok = false;
-                    break;
-                }
-                uint8_t *a = smem + st * Shape::STAGE, *b = a + ET_A_BYTES;
-                if (lane == 0) {
+        if (elect_one()) {
+            uint32_t fill = 0;  // number of the fill: stage fill % STAGES
+            bool ok = true;
+            auto freed = [&](uint32_t f) -> bool { return mbar_wait_bounded(&bar_free[f % STAGES], (f / STAGES) & 1u); };
+            for (int idx = blockIdx.x; idx < total && ok; idx += gridDim.x) {
+                if (!cur.seek(s_first, p, n_tiles, idx)) break;
+                for (int ks = 0; ks < k_steps; ++ks, ++fill) {
+                    const uint32_t st = fill % STAGES;
+                    if (fill >= STAGES && (*abort_flag != 0 || !freed(fill - STAGES))) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t *a = smem + st * Shape::STAGE, *b = a + ET_A_BYTES;
                     mbar_arrive_expect_tx(&bar_full[st], UP ? Shape::B_BYTES : Shape::STAGE);
                     if (UP) {
                         tma_load_4d(b, &map_w, &bar_full[st], ks * ET_K, cur.n * (BN / 2), 0, cur.e);
@@ -140,16 +148,14 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     }
                 }
             }
-        }
-        if (!ok) {
-            if (lane == 0) {
+            if (!ok) {
                 timed_out();
                 // copies already issued land before the CTA's memory is released
                 for (uint32_t f = fill > STAGES ? fill - STAGES : 0; f < fill; ++f)
                     mbar_wait_bounded(&bar_full[f % STAGES], (f / STAGES) & 1u, 100000000ull);
             }
-            __syncwarp();
         }
+        __syncwarp();
     } else if (warp == 1) {
         // =============== products ===================================================================
         if (elect_one()) {
@@ -185,28 +191,23 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         __syncwarp();
     } else if (UP && warp >= 6) {
         // =============== tokens =====================================================================
-        // 8 threads fetch the 128 bytes a token has in a step; a thread serves 8 tokens.  A step is handed over
-        // once the LAG of its own steps behind it have been asked for.
-        constexpr int LAG = STAGES / 2 - 1;
-        const uint32_t odd = tid >= ET_THREADS + ET_GATHER / 2;
-        const int pt = (tid - ET_THREADS) & (ET_GATHER / 2 - 1), chunk = pt & 7, r0 = pt >> 3;
-        uint32_t fill = 0, mine = 0;  // steps, and those of this half: its step k is number 2 k + odd
+        // 8 threads fetch the 128 bytes a token has in a step.  Each group of warps takes every GROUPS-th step and waits
+        // for its copies, so as many steps are on their way as there are groups.
+        constexpr int GROUPS = ET_GROUPS<STAGES>, GT = ET_GATHER / GROUPS, PER = ET_M * 8 / GT, ROWS = GT / 8;
+        const uint32_t group = (uint32_t)(tid - ET_THREADS) / GT;
+        const int pt = (tid - ET_THREADS) % GT, chunk = pt & 7, r0 = pt >> 3;
+        uint32_t fill = 0;
         bool ok = true;
-        auto hand_over = [&](uint32_t k) {
-            fence_proxy_async_smem();  // this thread's copies, before the products read them
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_full[(2 * k + odd) % STAGES]);
-        };
         for (int idx = blockIdx.x; idx < total && ok; idx += gridDim.x) {
             if (!cur.seek(s_first, p, n_tiles, idx)) break;
-            const __nv_bfloat16 *src[8];
+            const __nv_bfloat16 *src[PER];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int m = cur.m0 + r0 + 16 * i;  // nobody reads the results of rows behind the expert's last
+            for (int i = 0; i < PER; ++i) {
+                const int m = cur.m0 + r0 + ROWS * i;  // nobody reads the results of rows behind the expert's last
                 src[i] = m < cur.m_hi ? static_cast<const __nv_bfloat16 *>(p.a) + (long long)(p.slot[m] / p.top) * p.K + chunk * 8 : nullptr;
             }
             for (int ks = 0; ks < k_steps; ++ks, ++fill) {
-                if ((fill & 1u) != odd) continue;
+                if (fill % GROUPS != group) continue;
                 const uint32_t st = fill % STAGES, round = fill / STAGES;
                 if (round > 0 && !warp_wait(&bar_free[st], (round - 1) & 1u)) {
                     ok = false;
@@ -215,24 +216,19 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 const uint32_t base = smem_u32(smem + st * Shape::STAGE);
                 const int bytes = ks * ET_K + chunk * 8 < p.K ? 16 : 0;  // zeros behind the last channel
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = r0 + 16 * i;
+                for (int i = 0; i < PER; ++i) {
+                    const int r = r0 + ROWS * i;
                     if (src[i])
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(base + r * 128 + ((chunk ^ (r & 7)) << 4)),
                                      "l"(bytes ? src[i] + ks * ET_K : src[i]), "r"(bytes)
                                      : "memory");
                 }
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                if (mine >= (uint32_t)LAG) {
-                    asm volatile("cp.async.wait_group %0;" ::"n"(LAG) : "memory");
-                    hand_over(mine - LAG);
-                }
-                ++mine;
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                fence_proxy_async_smem();  // this thread's copies, before the products read them
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_full[st]);
             }
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (ok)
-            for (uint32_t k = mine > (uint32_t)LAG ? mine - LAG : 0; k < mine; ++k) hand_over(k);
         if (!ok && lane == 0 && *abort_flag == 0) timed_out();
         __syncwarp();
     } else {
@@ -247,7 +243,7 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const bool have = m < cur.m_hi;
             const float s = UP && have ? p.scale[m] : 0.f;
             const int n0 = cur.n * (UP ? BN / 2 : BN);
-            __nv_bfloat16 *out = static_cast<__nv_bfloat16 *>(p.out) + (long long)(UP ? m : (have ? p.slot[m] : 0)) * p.N;
+            const int to = UP ? m : (have ? p.slot[m] : 0);  // this row's place in out
             const uint32_t buf = tile & 1u;
             if (!warp_wait(&bar_acc[buf], (tile >> 1) & 1u)) {
                 if (lane == 0 && *abort_flag == 0) timed_out();
@@ -255,33 +251,47 @@ experts_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
             tc_fence_after();
             const uint32_t acc = tmem + buf * BN + lane_sel;
+            // 64 results of the warp's 32 rows at a time, turned in shared memory (16-byte pieces, swizzled by row): a
+            // store instruction then writes 128 bytes of four rows instead of 16 bytes of 32
+            uint8_t *turn = s_out + q * 32 * 128;
 #pragma unroll 1
-            for (int c = 0; c < (UP ? BN / 2 : BN); c += 32) {
+            for (int c = 0; c < (UP ? BN / 2 : BN); c += 64) {
                 if (n0 + c >= p.N) break;  // uniform over the CTA
-                __syncwarp();              // the loads below are warp-wide
-                float v[32];
-                if (UP) {
-                    float u[32];
-                    tmem_ld32x2(acc + c, v, acc + BN / 2 + c, u);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] = Fn<__nv_bfloat16>::silu(s * v[i]) * (s * u[i]);
-                } else {
-                    tmem_ld32(acc + c, v);
-                }
-                if (!have) continue;
+                for (int half = 0; half < 64; half += 32) {
+                    float v[32];
+                    if (UP) {
+                        float u[32];
+                        tmem_ld32x2(acc + c + half, v, acc + BN / 2 + c + half, u);
 #pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    const int n = n0 + c + i;
-                    if (vec) {
-                        if (n < p.N)
-                            *reinterpret_cast<uint4 *>(out + n) = make_uint4(pack_bf16x2(v[i], v[i + 1]), pack_bf16x2(v[i + 2], v[i + 3]),
-                                                                             pack_bf16x2(v[i + 4], v[i + 5]), pack_bf16x2(v[i + 6], v[i + 7]));
+                        for (int i = 0; i < 32; ++i) v[i] = Fn<__nv_bfloat16>::silu(s * v[i]) * (s * u[i]);
                     } else {
+                        tmem_ld32(acc + c + half, v);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; i += 8)
+                        *reinterpret_cast<uint4 *>(turn + lane * 128 + ((((half + i) / 8) ^ (lane & 7)) << 4)) =
+                            make_uint4(pack_bf16x2(v[i], v[i + 1]), pack_bf16x2(v[i + 2], v[i + 3]), pack_bf16x2(v[i + 4], v[i + 5]),
+                                       pack_bf16x2(v[i + 6], v[i + 7]));
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = i * 4 + (lane >> 3), n = n0 + c + (lane & 7) * 8;
+                    const int place = __shfl_sync(0xffffffffu, have ? to : -1, r);
+                    const uint4 w = *reinterpret_cast<const uint4 *>(turn + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+                    if (place < 0) continue;
+                    __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(p.out) + (long long)place * p.N + n;
+                    if (vec) {
+                        if (n < p.N) *reinterpret_cast<uint4 *>(dst) = w;
+                    } else {
+                        const uint32_t e[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                         for (int k = 0; k < 8; ++k)
-                            if (n + k < p.N) out[n + k] = __float2bfloat16_rn(v[i + k]);
+                            if (n + k < p.N) *reinterpret_cast<uint16_t *>(dst + k) = (uint16_t)(e[k >> 1] >> ((k & 1) * 16));
                     }
                 }
+                __syncwarp();  // read, before the next results are put there
             }
             tc_fence_before();
             __syncwarp();
@@ -307,11 +317,12 @@ static cudaError_t et_launch(const ExpertParams &p, cudaStream_t s, int *rc) {
     const int box[4] = {ET_K, UP ? BN / 2 : BN, 1, 1};
     *rc = make_tensor_map(&mw, p.w, 4, dims, strides, box);
     if (*rc != NCKV_OK) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(experts_tc_kernel<UP, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, EtShape<BN>::SMEM);
+    using Shape = EtShape<BN>;
+    const cudaError_t e = cudaFuncSetAttribute(experts_tc_kernel<UP, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::SMEM);
     if (e != cudaSuccess) return e;
     const long long tiles = ((long long)p.R / ET_M + p.E) * ((p.N + BN / halves - 1) / (BN / halves));
     const int grid = tiles < sm_count() ? (int)tiles : sm_count();
-    experts_tc_kernel<UP, BN><<<grid, ET_THREADS + (UP ? ET_GATHER : 0), EtShape<BN>::SMEM, s>>>(ma, mw, p);
+    experts_tc_kernel<UP, BN><<<grid, ET_THREADS + (UP ? ET_GATHER : 0), Shape::SMEM, s>>>(ma, mw, p);
     return cudaGetLastError();
 }
 
