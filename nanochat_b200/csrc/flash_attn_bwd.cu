@@ -152,9 +152,10 @@ struct BvShared {  // behind the operand tiles of the dK/dV kernel
     uint64_t bar_own, bar_walk[BU_RING], bar_s[2], bar_p[2], bar_d[2];
     uint32_t tmem_slot;
     int abort_flag;
-    // the walked queries' values, one per accumulator column: -lse * log2(e) and delta / sqrt(D)
-    alignas(16) float neg_lse2[2][BU];
-    alignas(16) float delta_s[2][BU];
+    // the walked queries' values, one per accumulator column of a warp: -lse * log2(e) and delta / sqrt(D).  Every warp keeps
+    // its own copy, so that the eight need not meet at a barrier in every unit
+    alignas(16) float neg_lse2[BT_EW_THREADS / 32][BU / 2];
+    alignas(16) float delta_s[BT_EW_THREADS / 32][BU / 2];
 };
 constexpr int BV_SMEM_BYTES = 2 * BT_TILE_BYTES + BU_RING * 2 * BU_TILE_BYTES + (int)sizeof(BvShared);
 
@@ -298,6 +299,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
         bool aborted = false;
         auto warp_wait = [&](uint64_t *bar, uint32_t parity) -> bool {
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;  // all lanes once, then one lane polls
             int ok = 1;
             if ((tid & 31) == 0) ok = mbar_wait_bounded(bar, parity, BT_WAIT_LIMIT) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -306,52 +308,45 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         };
         const float2 scale_log2_2 = make_float2(p.scale_log2, p.scale_log2), scale_2 = make_float2(p.scale, p.scale);
         const float2 zero_2 = make_float2(0.f, 0.f);
-        // threads 0-63 fetch -lse * log2(e), threads 64-127 delta / sqrt(D), of one of a unit's queries for everybody,
-        // one unit ahead so that the load is not on the path
+        // a lane fetches the two values of one of its warp's 32 queries, one unit ahead so that the loads are not on the path
+        const int col0 = half * 32;
         int head = 0, in_head = 0;  // of the unit whose values are fetched next: u / per_head, u % per_head
-        auto fetch = [&]() -> float {
-            float mine = 0.f;
-            if (tid < 2 * BU && head < rep) {
-                const int hq = hkv * rep + head, tq = (u_lo + in_head) * BU + (tid & (BU - 1));
-                mine = tid < BU ? -INFINITY : 0.f;  // a query past the end: P = 2^-inf = 0
+        auto fetch = [&]() -> float2 {
+            float2 mine = make_float2(-INFINITY, 0.f);  // lse and delta; a query past the end: P = 2^-inf = 0
+            if (head < rep) {
+                const int hq = hkv * rep + head, tq = (u_lo + in_head) * BU + col0 + (tid & 31);
                 if (tq < p.T) {
                     const long long o = ((long long)b * p.Hq + hq) * p.T + tq;
-                    if (tid < BU) {
-                        const float l = p.lse[o];
-                        mine = l == -INFINITY ? -INFINITY : -l * 1.4426950408889634f;
-                    } else {
-                        mine = p.delta[o] * p.scale;
-                    }
+                    mine.x = p.lse[o];
+                    mine.y = p.delta[o];
                 }
             }
             if (++in_head == per_head) { in_head = 0; ++head; }
             return mine;
         };
-        float mine = fetch();
+        float2 mine = fetch();
         int cur_in_head = 0;  // u % per_head of the current unit
         for (int u = 0; u < n_units; ++u) {
             const int q0 = (u_lo + cur_in_head) * BU;
             if (++cur_in_head == per_head) cur_in_head = 0;
             const int buf = u & 1;
-            const float mine_next = fetch();  // unit u + 1 (nothing past the last unit)
-            // (all eight warps take the same decision here: they meet at a named barrier right below)
+            const float2 mine_next = fetch();  // unit u + 1 (nothing past the last unit)
             if (!warp_wait(&sh.bar_s[buf], (uint32_t)(u >> 1) & 1u)) {
                 timed_out();
                 aborted = true;
                 break;
             }
             tc_fence_after();
-            if (tid < BU) sh.neg_lse2[buf][tid] = mine;
-            else if (tid < 2 * BU) sh.delta_s[buf][tid - BU] = mine;
-            asm volatile("bar.sync 1, 256;" ::: "memory");  // the eight elementwise warps
+            sh.neg_lse2[warp][tid & 31] = mine.x == -INFINITY ? -INFINITY : -mine.x * 1.4426950408889634f;  // (the values before have been read: the warp met ahead of its arrival on bar_p)
+            sh.delta_s[warp][tid & 31] = mine.y * p.scale;
+            __syncwarp();
             // only units on the diagonal or at the window's edge need masking: this key is seen by the unit's
             // queries [c_lo, c_hi)
             const bool edge = (q0 < k0 + BT - 1) || (p.window_left >= 0 && q0 + BU - 1 - k0 > p.window_left);
             const int c_lo = kp - q0;
             const int c_hi = p.window_left >= 0 ? kp + p.window_left - q0 + 1 : BU;
-            const int col0 = half * 32;
             const uint32_t t_s = tmem_base + (uint32_t)buf * 128 + lane_sel + col0;
-            const float *nls = &sh.neg_lse2[buf][col0], *dls = &sh.delta_s[buf][col0];
+            const float *nls = sh.neg_lse2[warp], *dls = sh.delta_s[warp];
             // two copies of the loop: the masked one only runs for the few units that need it
             auto chunk = [&](auto masked) {
                 constexpr bool MASKED = decltype(masked)::value;
@@ -554,6 +549,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
         bool aborted = false;
         auto warp_wait = [&](uint64_t *bar, uint32_t parity) -> bool {
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;  // all lanes once, then one lane polls
             int ok = 1;
             if ((tid & 31) == 0) ok = mbar_wait_bounded(bar, parity, BT_WAIT_LIMIT) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
