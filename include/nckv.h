@@ -423,6 +423,8 @@ NCKV_API int nckv_glue_ve_gate(const void *v, int64_t v_row_stride, const void *
  *   updated).  x_out must not alias x when mix is given.
  * nckv_silu_mul: rows [gate | up] of 2F -> silu(gate) * up.  nckv_tanh_split: tanh(z), fp32 or bf16 [hi | lo].
  * nckv_softcap: z = cap * tanh(z / cap) in place.
+ * nckv_linear_cap: out (R, N) = cap * tanh(x w^T / cap) in one launch, x (R, K) and w (N, K) packed bf16, fp32 sums and
+ *   results; K a multiple of 8, operands 16-byte aligned.  `status` receives NCKV_ST_TIMEOUT.
  * nckv_hyper_norm: S residual streams (rows, S, W): x_t' = sum_s mix[s, t] x_s + out[t] * (sum of the `parts`
  *   rows of y), or table[token] in all of them; h = layer norm (mean taken off, weight, no bias) of
  *   sum_t in[t] x_t' (in null: the plain sum).  x_out may be x, or null.  S <= 8.
@@ -471,6 +473,7 @@ NCKV_API int nckv_resid_norm(const float *x, const void *y, int y_f32, const flo
 NCKV_API int nckv_silu_mul(const void *gate_up, void *out, int64_t rows, int F, int f32, void *stream);
 NCKV_API int nckv_tanh_split(const float *z, void *out, int64_t rows, int R, int f32, void *stream);
 NCKV_API int nckv_softcap(float *z, int64_t n, float cap, void *stream);
+NCKV_API int nckv_linear_cap(const void *x, const void *w, float *out, int R, int N, int K, float cap, int32_t *status, void *stream);
 NCKV_API int nckv_rms_rope_append(const void *q, const void *k, const void *v, int64_t q_stride, int64_t k_stride, int64_t v_stride,
                       const float *q_weight, const float *k_weight, const float *cos_sin, const int32_t *cache_seqlens,
                       void *q_out, void *k_cache, void *v_cache, int64_t k_batch_stride, int64_t k_token_stride,

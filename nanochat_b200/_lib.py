@@ -77,6 +77,7 @@ SIGNATURES = {
     "nckv_silu_mul": (c_int, [c_void_p, c_void_p, c_i64, c_int, c_int, c_void_p]),
     "nckv_tanh_split": (c_int, [c_void_p, c_void_p, c_i64, c_int, c_int, c_void_p]),
     "nckv_softcap": (c_int, [c_void_p, c_i64, c_float, c_void_p]),
+    "nckv_linear_cap": (c_int, [c_void_p] * 3 + [c_int] * 3 + [c_float, c_void_p, c_void_p]),
     "nckv_rms_rope_append": (c_int, [c_void_p] * 3 + [c_i64] * 3 + [c_void_p] * 7 + [c_i64] * 4 + [c_int] * 11 +
                              [c_float, c_float, c_int, c_void_p, c_void_p]),
     "nckv_hyper_norm": (c_int, [c_void_p] * 3 + [c_int, c_void_p, c_int] + [c_void_p] * 6 + [c_int] * 3 + [c_float, c_int, c_void_p]),

@@ -134,7 +134,8 @@ class Sipadra(HybridDecoder):
                 n = len(logits_at)
                 x, y = self.pick(x, B, T, logits_at), self.pick(y, B, T, logits_at)
             _, h, _ = mo.resid_norm(x, y, w, eps=cfg.eps, dtype=self.dtype, B=B, T=n, final_weight=self.final_norm)
-            logits = mo.product(h, self.embed, f32_out=True)
             if cfg.logit_softcap is not None:
-                mo.softcap(logits, cfg.logit_softcap)
+                logits = mo.capped_product(h, self.embed, cfg.logit_softcap)
+            else:
+                logits = mo.product(h, self.embed, f32_out=True)
         return logits.view(B, n, -1)
