@@ -276,7 +276,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     } else if (issuer_warp) {
         // =============== one thread feeds the tensor core ==========================================
         // tcgen05.mma / tcgen05.commit are single-thread instructions and an mbarrier poll by 32 lanes
-        // is 32 polls, one after the other: lane 0 runs this role alone.
+        // is 32 polls, one after the other: one elected thread runs this role alone.
         if (elect_one()) {
             // Descriptors differ only in the start-address field (address >> 4 in the low 14 bits),
             // so they are built once and advanced by adding the byte offset >> 4.
