@@ -12,14 +12,15 @@
 // a token has the same bits however the sequence was cut into calls (see the segments below for the
 // one exception, which is at fp32 rounding level).
 //
-// Mapping.  A CTA owns up to 128 value columns of one (row, head, segment).  A warp owns VG*8 of them:
-// lane = vg * KG + kg holds key channels {4 KG i + 4 kg + j : i < U, j < 4} of columns {8 vg + c : c < 8}.
+// Mapping.  A CTA owns up to 128 value columns of one (row, head, segment).  A warp owns VG*CL of them (CL = REC_LANE):
+// lane = vg * KG + kg holds key channels {4 KG i + 4 kg + j : i < U, j < 4} of columns {CL vg + c : c < CL}.
 // Pairs of key channels are the two halves of packed fp32 instructions; a step is three of them per
 // pair and column.  Tokens run in batches of 4: their partial outputs are summed over the KG lanes
-// together (a reduce-scatter that leaves a lane 2 or 4 columns of one token), so the latency of the
+// together (a reduce-scatter that leaves a lane 1 to 4 columns of one token), so the latency of the
 // shuffles is paid once per batch.  Batches are padded with tokens that leave the state as it is
-// (k = 0, w = 1).  Per warp and token 3 U + 2 16-byte shared-memory loads stand against 48 U packed
-// multiply-adds: the fp32 pipe is the bound, shared memory and the issue slots are just below it.  Tokens are staged C at a time through two buffers
+// (k = 0, w = 1).  Per warp and token 3 U + CL / 4 16-byte shared-memory loads stand against 6 CL U packed
+// multiply-adds; with one CTA per head the number of warps per scheduler, which hide the latencies of these loads and
+// of the shuffles, is the bound, the fp32 pipe and the issue slots lie below it.  Tokens are staged C at a time through two buffers
 // (converted, activated and exponentiated once per head on the way, by all warps evenly); the next
 // chunk's bytes wait in registers meanwhile.  8 threads normalise, gate and store a token of the
 // chunk before.
@@ -64,6 +65,13 @@ struct RecurrentParams {
 };
 
 constexpr int REC_COLS = 128;  // value columns per CTA
+constexpr int REC_TOKENS = 32; // tokens staged at a time, at most
+// Value columns of a lane.  Four: twice the warps of eight for the same columns, which hide each other's latencies (with
+// eight a scheduler had one or two warps and issued in 40 percent of its cycles): per-channel decay, 8 x 2048 tokens, 24
+// heads of 64 x 64, 622 -> 534 us; per-head decay, 1 x 8192, 16 heads of 128 x 128, 560 -> 512.  Eight where a lane has four key
+// channels and a constant decay, which leaves the least work per shared-memory load: 8 x 2048, 12 heads of 64 x 128, 457 us
+// against 463.
+template <int U, bool CHANNEL> constexpr int REC_LANE = !CHANNEL && U == 1 ? 8 : 4;
 constexpr int REC_BATCH = 4;   // tokens whose outputs are reduced together
 constexpr int REC_MAXQ = 2;    // 4-element pieces a thread stages per vector and chunk
 
@@ -168,8 +176,8 @@ template <int BIT, int LEN> __device__ __forceinline__ int reduce_scatter(float 
 
 // CHANNEL: decay per token and key channel, bonus form.  OUT: false in the first pass over segments.
 template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC>
-__global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(const RecurrentParams p) {
-    constexpr int TB = REC_BATCH, VG = 32 / KG, KP = 4 * KG * U, KQ = KP / 4, WC = 8 * VG;  // WC: columns per warp
+__global__ void __launch_bounds__(REC_COLS / (32 * REC_LANE<U, CHANNEL> / KG) * 32) recurrent_kernel(const RecurrentParams p) {
+    constexpr int TB = REC_BATCH, VG = 32 / KG, KP = 4 * KG * U, KQ = KP / 4, CL = REC_LANE<U, CHANNEL>, WC = CL * VG;  // WC: columns per warp
     constexpr int NB = KQ > 32 ? KQ / 32 : 1;                               // partial bonus sums per token
     const int NT = blockDim.x, NW = NT >> 5;
     const int VP = NW * WC, VQ = VP / 4;
@@ -187,8 +195,8 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
     const int off_v = C * KP, off_q = off_v + C * VP, off_w = off_q + (OUT ? C * KP : 0), off_b = off_w + (CHANNEL ? C * KP : 0);
 
     // ---- this lane's part of the state: all loads in flight together ----------------------------------
-    float2 S[U * 2][8];  // [pair of key channels][column]
-    const int v0 = warp * WC + vg * 8;
+    float2 S[U * 2][CL];  // [pair of key channels][column]
+    const int v0 = warp * WC + vg * CL;
     const long long state_base = (((long long)seg * p.B + b) * p.H + h) * (long long)Dk * p.Dv + col0;
     {
         const float *src = p.state_in + state_base;
@@ -197,7 +205,7 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
         for (int i = 0; i < U * 4; ++i) {
             const int kc = (i >> 2) * 4 * KG + kg * 4 + (i & 3);
 #pragma unroll
-            for (int c = 0; c < 8; c += 4) {
+            for (int c = 0; c < CL; c += 4) {
                 const float4 f = load_quad<VEC>(src + (long long)kc * p.Dv + v0 + c, have && kc < Dk && v0 + c < Dv, Dv - v0 - c).w;
                 const float e[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
@@ -304,12 +312,12 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
         const float *bk = buf + kg * 4, *bv = buf + off_v + v0;
 #pragma unroll 1
         for (int tb = 0; tb < n; tb += TB) {
-            float o[TB * 8];  // [token][column], partial sums over this lane's key channels
+            float o[TB * CL];  // [token][column], partial sums over this lane's key channels
 #pragma unroll
             for (int tt = 0; tt < TB; ++tt) {
                 const int t = tb + tt;
                 float2 k2[U * 2], w2[U * 2], q2[OUT ? U * 2 : 1];
-                float vv[8];
+                float vv[CL];
 #pragma unroll
                 for (int i = 0; i < U; ++i) {
                     float4 f = *reinterpret_cast<const float4 *>(bk + t * KP + i * 4 * KG);
@@ -330,7 +338,7 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
                     }
                 }
 #pragma unroll
-                for (int c = 0; c < 8; c += 4) {
+                for (int c = 0; c < CL; c += 4) {
                     const float4 f = *reinterpret_cast<const float4 *>(bv + t * VP + c);
                     vv[c] = f.x; vv[c + 1] = f.y; vv[c + 2] = f.z; vv[c + 3] = f.w;
                 }
@@ -339,7 +347,7 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
                     for (int i = 0; i < U * 2; ++i) prod2[i] = fmul2(prod2[i], w2[i]);
                 }
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
+                for (int c = 0; c < CL; ++c) {
                     const float2 vd = make_float2(vv[c], vv[c]);
                     float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
@@ -348,13 +356,13 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
                         S[i][c] = ffma2(w2[i], S[i][c], fmul2(k2[i], vd));
                         if (OUT && !CHANNEL) acc = i ? ffma2(q2[i], S[i][c], acc) : fmul2(q2[i], S[i][c]);
                     }
-                    if (OUT) o[tt * 8 + c] = acc.x + acc.y;
+                    if (OUT) o[tt * CL + c] = acc.x + acc.y;
                 }
             }
             if (OUT) {
-                const int first = reduce_scatter<KG / 2, TB * 8>(o, kg);
-                constexpr int HELD = TB * 8 / KG;  // 4 or 2 columns of one token
-                const int t = tb + first / 8, col = v0 + first % 8;
+                const int first = reduce_scatter<KG / 2, TB * CL>(o, kg);
+                constexpr int HELD = TB * CL / KG;  // columns of one token
+                const int t = tb + first / CL, col = v0 + first % CL;
                 float bonus = 0.f;
                 if (CHANNEL) {
                     bonus = buf[off_b + t * 4];
@@ -415,7 +423,7 @@ __global__ void __launch_bounds__(REC_COLS / (256 / KG) * 32) recurrent_kernel(c
         for (int i = 0; i < U * 4; ++i) {
             const int kc = (i >> 2) * 4 * KG + kg * 4 + (i & 3);
 #pragma unroll
-            for (int c = 0; c < 8; c += 4) {
+            for (int c = 0; c < CL; c += 4) {
                 float e[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) e[j] = (i & 1) ? S[i >> 1][c + j].y : S[i >> 1][c + j].x;
@@ -555,7 +563,7 @@ static cudaError_t rec_step_launch(RecurrentParams p, cudaStream_t s) {
 
 template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC>
 static cudaError_t rec_launch_one(RecurrentParams p, cudaStream_t s) {
-    constexpr int TB = REC_BATCH, WC = 256 / KG, KP = 4 * KG * U;
+    constexpr int TB = REC_BATCH, WC = 32 * REC_LANE<U, CHANNEL> / KG, KP = 4 * KG * U;
     const int cols = p.Dv < REC_COLS ? p.Dv : REC_COLS;
     int NW = (cols + WC - 1) / WC;
     while (REC_MAXQ * NW * 32 < TB * (KP / 4)) ++NW;  // room to stage a batch (wide keys, few value columns)
@@ -563,7 +571,9 @@ static cudaError_t rec_launch_one(RecurrentParams p, cudaStream_t s) {
     int C = REC_MAXQ * NT / (KP / 4);
     const int Cv = REC_MAXQ * (NT / (VP / 4));
     if (Cv < C) C = Cv;
-    if (C > 16) C = 16;
+    if (C > REC_TOKENS) C = REC_TOKENS;
+    const int most = (p.seg_len + TB - 1) / TB * TB;  // a short call stages no more than it has
+    if (C > most) C = most;
     p.C = C -= C % TB;
     p.n_cols = (p.Dv + VP - 1) / VP;
     const size_t smem = sizeof(float) * (2ull * KP + VP + 2ull * C * (KP + VP + (OUT ? KP : 0) + (CHANNEL ? KP : 0) + (OUT && CHANNEL ? 4 : 0)) +
