@@ -379,6 +379,8 @@ NCKV_API int nckv_flash_attn_bwd(const void *q, const void *k, const void *v, co
  *     out_norm = bf16(y * rsqrt(mean(y^2) + eps))   (norm, gpt.py:42-43)           gpt.py:149-150, 468
  * out_sum (optional, needs add) receives a, out_x (optional) receives y, out_norm (optional) the
  * normalised row; the fp32 sum of squares is accumulated in the order of torch's row kernel.
+ * nckv_glue_mix_norm_at: the same with the scalars on the device, where the kernel reads them when it runs: bf16, or fp32
+ * (rounded to bf16, as the eager multiply does) where bit 0 (resid), 1 (x0) or 2 (backout) of f32_mask is set.
  * nckv_glue_relu_sq: out = bf16(max(h, 0)^2) over n elements (n % 8 == 0), MLP.forward gpt.py:136.
  * nckv_glue_ve_gate: v_out = bf16(v + bf16(bf16(3 * bf16(sigmoid(gate_lin))) * ve)) with v, ve (rows, Hkv, D)
  * and gate_lin (rows, Hkv) the output of the gate's linear layer: the value residual of gpt.py:92-95.  v may have
@@ -389,6 +391,9 @@ NCKV_API int nckv_flash_attn_bwd(const void *q, const void *k, const void *v, co
 NCKV_API int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
                        void *out_x, void *out_norm, int rows, int C, int mode, float resid_lambda, float x0_lambda,
                        float backout_lambda, float eps, void *stream);
+NCKV_API int nckv_glue_mix_norm_at(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
+                       void *out_x, void *out_norm, int rows, int C, int mode, const void *resid_lambda,
+                       const void *x0_lambda, const void *backout_lambda, int f32_mask, float eps, void *stream);
 NCKV_API int nckv_glue_relu_sq(const void *h, void *out, int64_t n, void *stream);
 NCKV_API int nckv_glue_logit_cap(const void *z, int64_t z_row_stride, float *out, int64_t rows, int cols, float cap, void *stream);
 NCKV_API int nckv_glue_ve_gate(const void *v, int64_t v_row_stride, const void *gate_lin, const void *ve, void *v_out, int rows, int Hkv, int D,

@@ -45,6 +45,7 @@ SIGNATURES = {
     "nckv_p2p_wait_combine": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                       ctypes.c_uint64, c_void_p]),
     "nckv_glue_mix_norm": (c_int, [c_void_p] * 7 + [c_int] * 3 + [c_float] * 4 + [c_void_p]),
+    "nckv_glue_mix_norm_at": (c_int, [c_void_p] * 7 + [c_int] * 3 + [c_void_p] * 3 + [c_int, c_float, c_void_p]),
     "nckv_glue_relu_sq": (c_int, [c_void_p, c_void_p, c_i64, c_void_p]),
     "nckv_glue_logit_cap": (c_int, [c_void_p, c_i64, c_void_p, c_i64, c_int, c_float, c_void_p]),
     "nckv_glue_ve_gate": (c_int, [c_void_p, c_i64] + [c_void_p] * 3 + [c_int] * 3 + [c_void_p]),

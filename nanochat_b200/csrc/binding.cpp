@@ -128,9 +128,10 @@ bool row_tensor(const Tensor &t, const Tensor &like) {
 
 using Three = std::tuple<std::optional<Tensor>, std::optional<Tensor>, std::optional<Tensor>>;
 
-std::optional<Three> glue_mix_norm(const Tensor &x, const std::optional<Tensor> &add, const std::optional<Tensor> &x0,
-                                   const std::optional<Tensor> &x_backout, double resid_lambda, double x0_lambda, double backout_lambda,
-                                   bool want_sum, bool want_x, bool want_norm, double eps) {
+// launch(pointers of x, add, x0, x_backout, sum, y, norm, rows, channels, mode, stream) does the rest
+template <typename Launch>
+std::optional<Three> mix_norm(const Tensor &x, const std::optional<Tensor> &add, const std::optional<Tensor> &x0,
+                              const std::optional<Tensor> &x_backout, bool want_sum, bool want_x, bool want_norm, const Launch &launch) {
     if (!x.is_cuda() || x.dim() == 0 || x.numel() == 0 || !row_tensor(x, x)) return std::nullopt;
     for (const std::optional<Tensor> *t : {&add, &x0, &x_backout})
         if (*t && !row_tensor(**t, x)) return std::nullopt;
@@ -144,10 +145,41 @@ std::optional<Three> glue_mix_norm(const Tensor &x, const std::optional<Tensor> 
     if (want_norm) norm = at::empty_like(x);
     auto ptr = [](const std::optional<Tensor> &t) { return t ? t->data_ptr() : nullptr; };
     const cudaStream_t s = at::cuda::getCurrentCUDAStream(x.device().index()).stream();
-    if (nckv_glue_mix_norm(x.data_ptr(), ptr(add), ptr(x0), ptr(x_backout), ptr(sum), ptr(y), ptr(norm), (int)rows, (int)C,
-                           x0 ? 1 : (x_backout ? 2 : 0), (float)resid_lambda, (float)x0_lambda, (float)backout_lambda, (float)eps, s) < 0)
+    if (launch(x.data_ptr(), ptr(add), ptr(x0), ptr(x_backout), ptr(sum), ptr(y), ptr(norm), (int)rows, (int)C, x0 ? 1 : (x_backout ? 2 : 0), s) < 0)
         return std::nullopt;
     return out;
+}
+
+std::optional<Three> glue_mix_norm(const Tensor &x, const std::optional<Tensor> &add, const std::optional<Tensor> &x0,
+                                   const std::optional<Tensor> &x_backout, double resid_lambda, double x0_lambda, double backout_lambda,
+                                   bool want_sum, bool want_x, bool want_norm, double eps) {
+    return mix_norm(x, add, x0, x_backout, want_sum, want_x, want_norm,
+                    [&](void *px, void *pa, void *p0, void *pb, void *ps, void *py, void *pn, int rows, int C, int mode, cudaStream_t s) {
+                        return nckv_glue_mix_norm(px, pa, p0, pb, ps, py, pn, rows, C, mode, (float)resid_lambda, (float)x0_lambda,
+                                                  (float)backout_lambda, (float)eps, s);
+                    });
+}
+
+// The same with the scalars (those of the mix that is asked for) as elements on the rows' device.
+std::optional<Three> glue_mix_norm_at(const Tensor &x, const std::optional<Tensor> &add, const std::optional<Tensor> &x0,
+                                      const std::optional<Tensor> &x_backout, const std::optional<Tensor> &resid_lambda,
+                                      const std::optional<Tensor> &x0_lambda, const std::optional<Tensor> &backout_lambda, bool want_sum,
+                                      bool want_x, bool want_norm, double eps) {
+    const void *at[3] = {};
+    int f32_mask = 0, i = 0;
+    for (const std::optional<Tensor> *t : {&resid_lambda, &x0_lambda, &backout_lambda}) {
+        if (*t) {
+            const bool f32 = (*t)->scalar_type() == at::kFloat;
+            if ((*t)->numel() != 1 || (*t)->device() != x.device() || (!f32 && (*t)->scalar_type() != at::kBFloat16)) return std::nullopt;
+            at[i] = (*t)->data_ptr();
+            f32_mask |= (int)f32 << i;
+        }
+        ++i;
+    }
+    return mix_norm(x, add, x0, x_backout, want_sum, want_x, want_norm,
+                    [&](void *px, void *pa, void *p0, void *pb, void *ps, void *py, void *pn, int rows, int C, int mode, cudaStream_t s) {
+                        return nckv_glue_mix_norm_at(px, pa, p0, pb, ps, py, pn, rows, C, mode, at[0], at[1], at[2], f32_mask, (float)eps, s);
+                    });
 }
 
 std::optional<Tensor> glue_relu_sq(const Tensor &h) {
@@ -165,5 +197,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("set_workspace", &set_workspace);
     m.def("kv_attention", &kv_attention);
     m.def("glue_mix_norm", &glue_mix_norm);
+    m.def("glue_mix_norm_at", &glue_mix_norm_at);
     m.def("glue_relu_sq", &glue_relu_sq);
 }

@@ -25,12 +25,26 @@ namespace nckv {
 constexpr int GLUE_THREADS = 128;  // 32 x 4, the block shape whose reduction order is reproduced
 constexpr int GLUE_MAX_VEC = 16;   // vectors of 4 channels per thread: C <= 8192
 
+struct GlueScalar {
+    const void *at;  // on the device, fp32 or bf16, or null
+    float value;     // without `at`
+    bool f32;
+};
+
 struct GlueRowParams {
     const uint2 *x, *add, *x0, *xb;
     uint2 *out_sum, *out_x, *out_norm;
-    float rl, xl, bl, eps;
+    GlueScalar rl, xl, bl;
+    float eps;
     int C, mode;  // mode 0: y = a, 1: lambda mix, 2: backout
 };
+
+// A parameter on the device is read there by every launch, so that its owner may write or replace it between any two,
+// replays of a graph included; rounded to bf16 as the eager multiply rounds it.
+__device__ __forceinline__ float scalar_value(const GlueScalar &s) {
+    if (!s.at) return s.value;
+    return s.f32 ? round_bf16(*static_cast<const float *>(s.at)) : __bfloat162float(*static_cast<const __nv_bfloat16 *>(s.at));
+}
 
 __device__ __forceinline__ void unpack4(const uint2 &v, float (&f)[4]) {
     f[0] = bf16lo(v.x); f[1] = bf16hi(v.x);
@@ -62,6 +76,7 @@ __global__ void __launch_bounds__(GLUE_THREADS) glue_row_kernel(const GlueRowPar
             if (p.mode != 0) in_second[k] = second[base + i];
         }
     }
+    const float rl = p.mode == 1 ? scalar_value(p.rl) : 0.f, second_l = p.mode == 1 ? scalar_value(p.xl) : p.mode == 2 ? scalar_value(p.bl) : 0.f;
     float y[NV][4];
     float acc = 0.f;
 #pragma unroll
@@ -82,8 +97,8 @@ __global__ void __launch_bounds__(GLUE_THREADS) glue_row_kernel(const GlueRowPar
                 unpack4(in_second[k], z);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    a[e] = p.mode == 1 ? round_bf16(__fadd_rn(round_bf16(__fmul_rn(p.rl, a[e])), round_bf16(__fmul_rn(p.xl, z[e]))))
-                                       : round_bf16(__fsub_rn(a[e], round_bf16(__fmul_rn(p.bl, z[e]))));
+                    a[e] = p.mode == 1 ? round_bf16(__fadd_rn(round_bf16(__fmul_rn(rl, a[e])), round_bf16(__fmul_rn(second_l, z[e]))))
+                                       : round_bf16(__fsub_rn(a[e], round_bf16(__fmul_rn(second_l, z[e]))));
             }
             if (p.out_x) p.out_x[base + i] = pack4(a);
 #pragma unroll
@@ -197,9 +212,9 @@ int nckv_glue_logit_cap(const void *z, int64_t z_row_stride, float *out, int64_t
     return NCKV_OK;
 }
 
-int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
-                       void *out_x, void *out_norm, int rows, int C, int mode, float resid_lambda, float x0_lambda,
-                       float backout_lambda, float eps, void *stream) {
+static int glue_mix_norm_impl(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
+                              void *out_x, void *out_norm, int rows, int C, int mode, nckv::GlueScalar resid_lambda,
+                              nckv::GlueScalar x0_lambda, nckv::GlueScalar backout_lambda, float eps, void *stream) {
     using namespace nckv;
     if (!x || rows <= 0 || (!out_x && !out_norm && !out_sum)) {
         set_error("glue_mix_norm: null pointer or non-positive row count");
@@ -235,6 +250,32 @@ int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const voi
     kernel<<<rows, GLUE_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(p);
     NCKV_CUDA_CHECK(cudaGetLastError());
     return NCKV_OK;
+}
+
+int nckv_glue_mix_norm(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
+                       void *out_x, void *out_norm, int rows, int C, int mode, float resid_lambda, float x0_lambda,
+                       float backout_lambda, float eps, void *stream) {
+    using nckv::GlueScalar;
+    return glue_mix_norm_impl(x, add, x0, x_backout, out_sum, out_x, out_norm, rows, C, mode, GlueScalar{nullptr, resid_lambda, true},
+                              GlueScalar{nullptr, x0_lambda, true}, GlueScalar{nullptr, backout_lambda, true}, eps, stream);
+}
+
+int nckv_glue_mix_norm_at(const void *x, const void *add, const void *x0, const void *x_backout, void *out_sum,
+                          void *out_x, void *out_norm, int rows, int C, int mode, const void *resid_lambda,
+                          const void *x0_lambda, const void *backout_lambda, int f32_mask, float eps, void *stream) {
+    using nckv::GlueScalar;
+    if ((mode == 1 && (!resid_lambda || !x0_lambda)) || (mode == 2 && !backout_lambda)) {
+        nckv::set_error("glue_mix_norm: mode %d lacks a scalar", mode);
+        return NCKV_E_ARG;
+    }
+    const void *at[3] = {resid_lambda, x0_lambda, backout_lambda};
+    for (int i = 0; i < 3; ++i)
+        if ((uintptr_t)at[i] & ((f32_mask >> i & 1) ? 3 : 1)) {
+            nckv::set_error("glue_mix_norm: misaligned scalar");
+            return NCKV_E_ARG;
+        }
+    return glue_mix_norm_impl(x, add, x0, x_backout, out_sum, out_x, out_norm, rows, C, mode, GlueScalar{resid_lambda, 0.f, (f32_mask & 1) != 0},
+                              GlueScalar{x0_lambda, 0.f, (f32_mask & 2) != 0}, GlueScalar{backout_lambda, 0.f, (f32_mask & 4) != 0}, eps, stream);
 }
 
 int nckv_glue_relu_sq(const void *h, void *out, int64_t n, void *stream) {

@@ -246,7 +246,7 @@ class GPT(nn.Module):
         # run the eager op sequence everywhere.
         self.fused_glue = True
         self.fused_qkv = True   # one [c_q; c_k; c_v] product per layer in the decode trunk where it is bit-identical
-        self._lambda_cache = None
+        self._lambda_cache = None  # stays empty: the scalars are read where they lie, in every pass
         self.rotary_seq_len = config.sequence_len * 10  # same over-allocation as gpt.py:195
         self.register_buffer("cos", torch.empty(0), persistent=False)
         self.register_buffer("sin", torch.empty(0), persistent=False)
@@ -343,7 +343,7 @@ class GPT(nn.Module):
         x_backout = None
         rope_tables = (self.cos, self.sin)
         if self.fused_glue and kv_cache is not None and x.is_cuda and x.dtype == torch.bfloat16 and \
-                (T == 1 or self._prompt_can_fuse(B)):
+                (T == 1 or self._prompt_can_fuse(B, x.device)):
             return self._head(self._trunk_fused(idx, x, kv_cache, rope_tables), logits_at)
         for i, block in enumerate(self.transformer.h):
             x = self.resid_lambdas[i] * x + self.x0_lambdas[i] * x0
@@ -355,13 +355,12 @@ class GPT(nn.Module):
             x = x - self.backout_lambda.to(x.dtype) * x_backout
         return self._head(rms(x), logits_at)
 
-    def _prompt_can_fuse(self, rows):
-        """The fused trunk reads the lambdas on the host once per version, which a stream capture does not allow and
-        inference tensors do not have, and it has a widest row; the eager trunk takes the rest."""
-        if rows == 0 or self.config.n_embd > ops.GLUE_MAX_C or self.resid_lambdas.is_inference():
-            return False
-        known = self._lambda_cache is not None and self._lambda_cache[0] == self._lambda_key()
-        return known or not torch.cuda.is_current_stream_capturing()
+    def _prompt_can_fuse(self, rows, device):
+        """The fused trunk has a widest row and rounds the lambdas as the eager multiply does for bf16 and fp32 ones on
+        the activations' device; the eager trunk takes the rest."""
+        return rows > 0 and self.config.n_embd <= ops.GLUE_MAX_C and all(
+            t.device == device and t.dtype in (torch.bfloat16, torch.float32)
+            for t in (self.resid_lambdas, self.x0_lambdas, self.backout_lambda))
 
     def _head(self, x, logits_at):
         """Soft-capped logits of normed activations (B, T, C), at the given places only if there are any given."""
@@ -372,20 +371,16 @@ class GPT(nn.Module):
             return ops.glue_logit_cap(z, self.config.vocab_size, 15.0)
         return 15 * torch.tanh(z[..., :self.config.vocab_size].float() / 15)
 
-    def _lambda_key(self):
-        return (self.resid_lambdas.data_ptr(), self.resid_lambdas._version, self.x0_lambdas._version,
-                self.backout_lambda._version, self.resid_lambdas.dtype)
-
-    def _lambdas(self):
-        """Host copies of the per-layer scalars, read once (a device read per step would synchronise),
-        rounded to bf16: the eager multiply converts a 0-dim parameter to the activation dtype before it
-        multiplies (and gpt.py:467 casts the backout lambda explicitly)."""
-        key = self._lambda_key()
-        if self._lambda_cache is None or self._lambda_cache[0] != key:
-            as_bf16 = lambda t: t.detach().to(torch.bfloat16).float()
-            self._lambda_cache = (key, as_bf16(self.resid_lambdas).tolist(), as_bf16(self.x0_lambdas).tolist(),
-                                  float(as_bf16(self.backout_lambda).item()))
-        return self._lambda_cache[1:]
+    def _lambdas(self, device):
+        """(mixing op, per-layer scalars for it): one-element views that the kernels read, so that a parameter may be
+        written or replaced between any two passes; numbers where a parameter is on another device.  They round to
+        bf16: the eager multiply converts a 0-dim parameter to the activation dtype before it multiplies (and
+        gpt.py:467 casts the backout lambda explicitly)."""
+        params = [t.detach().reshape(-1) for t in (self.resid_lambdas, self.x0_lambdas, self.backout_lambda)]
+        if all(t.device == device for t in params):
+            return ops.glue_mix_norm_at, *((t if t.dtype in (torch.bfloat16, torch.float32) else t.to(torch.bfloat16)).unbind()
+                                           for t in params)
+        return ops.glue_mix_norm, *(t.to(torch.bfloat16).float().tolist() for t in params)
 
     def _trunk_fused(self, idx, x, kv_cache, rope_tables):
         """The layer loop of ``forward`` over a cache with the elementwise glue fused, up to the last norm:
@@ -394,7 +389,7 @@ class GPT(nn.Module):
         one), instead of about a dozen eager launches.  Same matrix products, same roundings."""
         B, T = idx.shape
         C = x.size(-1)
-        resid, x0l, backout = self._lambdas()
+        mix, resid, x0l, (backout,) = self._lambdas(x.device)
         n_layer = self.config.n_layer
         backout_at = n_layer // 2
         x = x.contiguous()
@@ -403,8 +398,7 @@ class GPT(nn.Module):
         x_backout = None
         for i, block in enumerate(self.transformer.h):
             # the residual stream after layer backout_at is needed later: keep the sum when the add happens
-            x_sum, x, xn = ops.glue_mix_norm(x, add=pending, x0=x0, resid_lambda=resid[i], x0_lambda=x0l[i],
-                                             want_sum=(i == backout_at + 1))
+            x_sum, x, xn = mix(x, add=pending, x0=x0, resid_lambda=resid[i], x0_lambda=x0l[i], want_sum=(i == backout_at + 1))
             if i == backout_at + 1:
                 x_backout = x_sum
             attn = block.attn
@@ -428,9 +422,9 @@ class GPT(nn.Module):
             pending = block.mlp.c_proj(ops.glue_relu_sq(block.mlp.c_fc(xn)))
         if backout_at == n_layer - 1:  # only a one-layer model: the backout operand is the final sum itself
             x_backout, _, _ = ops.glue_mix_norm(x, add=pending, want_sum=True, want_x=False, want_norm=False)
-            _, _, xn = ops.glue_mix_norm(x_backout, x_backout=x_backout, backout_lambda=backout, want_x=False)
+            _, _, xn = mix(x_backout, x_backout=x_backout, backout_lambda=backout, want_x=False)
         else:
-            _, _, xn = ops.glue_mix_norm(x, add=pending, x_backout=x_backout, backout_lambda=backout, want_x=False)
+            _, _, xn = mix(x, add=pending, x_backout=x_backout, backout_lambda=backout, want_x=False)
         return xn
 
     @torch.inference_mode()

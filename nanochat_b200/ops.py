@@ -692,10 +692,29 @@ def glue_mix_norm(x, add=None, x0=None, x_backout=None, resid_lambda=1.0, x0_lam
     ``a = x (+ add)``; then ``resid_lambda * a + x0_lambda * x0`` (when ``x0`` is given) or
     ``a - backout_lambda * x_backout`` (when ``x_backout`` is given); then rms-norm.  Every step
     rounds to bf16 like the eager op it stands for.  Returns (a or None, y or None, norm or None)."""
-    name = "glue_mix_norm"
     done = _lib.native.glue_mix_norm(x, add, x0, x_backout, resid_lambda, x0_lambda, backout_lambda, want_sum, want_x, want_norm, eps)
     if done is not None:
         return done
+    return _mix_norm("glue_mix_norm", x, add, x0, x_backout, (float(resid_lambda), float(x0_lambda), float(backout_lambda)),
+                     want_sum, want_x, want_norm, eps)
+
+
+def glue_mix_norm_at(x, add=None, x0=None, x_backout=None, resid_lambda=None, x0_lambda=None, backout_lambda=None,
+                     want_sum=False, want_x=True, want_norm=True, eps=RMS_EPS):
+    """``glue_mix_norm`` with its scalars on the rows' device, one fp32 or bf16 element each: the kernel reads them
+    when it runs and rounds them to bf16, as the eager multiply by a parameter does."""
+    done = _lib.native.glue_mix_norm_at(x, add, x0, x_backout, resid_lambda, x0_lambda, backout_lambda, want_sum, want_x, want_norm, eps)
+    if done is not None:
+        return done
+    scalars = (resid_lambda, x0_lambda, backout_lambda)
+    for s in scalars:
+        if s is not None and (s.device != x.device or s.numel() != 1 or s.dtype not in (torch.float32, torch.bfloat16)):
+            raise RuntimeError("nckv::glue_mix_norm_at needs scalars of one fp32 or bf16 element each on the rows' device")
+    f32_mask = sum((s is not None and s.dtype == torch.float32) << i for i, s in enumerate(scalars))
+    return _mix_norm("glue_mix_norm_at", x, add, x0, x_backout, (*(_ptr(s) for s in scalars), f32_mask), want_sum, want_x, want_norm, eps)
+
+
+def _mix_norm(name, x, add, x0, x_backout, scalars, want_sum, want_x, want_norm, eps):
     C = x.size(-1)
     px = _rows(name, x, C)
     rows = x.numel() // C
@@ -705,11 +724,11 @@ def glue_mix_norm(x, add=None, x0=None, x_backout=None, resid_lambda=1.0, x0_lam
     out_norm = torch.empty_like(x) if want_norm else None
     idx = x.device.index
     with _device_guard(idx):
-        _lib.call("nckv_glue_mix_norm", px, _rows(name, add, C) if add is not None else None,
+        _lib.call("nckv_" + name, px, _rows(name, add, C) if add is not None else None,
                   _rows(name, x0, C) if x0 is not None else None,
                   _rows(name, x_backout, C) if x_backout is not None else None,
-                  _ptr(out_sum), _ptr(out_x), _ptr(out_norm), rows, C, mode, float(resid_lambda), float(x0_lambda),
-                  float(backout_lambda), float(eps), torch.cuda.current_stream(idx).cuda_stream)
+                  _ptr(out_sum), _ptr(out_x), _ptr(out_norm), rows, C, mode, *scalars, float(eps),
+                  torch.cuda.current_stream(idx).cuda_stream)
     return out_sum, out_x, out_norm
 
 
