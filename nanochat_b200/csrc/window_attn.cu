@@ -214,15 +214,19 @@ __global__ void __launch_bounds__(256) rms_rope_append_kernel(const RmsRopeParam
 // ------------------------------------------------------------------------------------------------
 // Both appends for heads of 128 channels that are rotated as a whole, in bf16: lane j of a half-warp holds channels
 // 4j .. 4j + 3 and 64 + 4j .. 64 + 4j + 3 of a head, the two sides of its rotation pairs.  The general kernels load
-// every pair twice, table entries one by one, and divide 64-bit indices per head row: 183 us against 88 us for
-// 8 x 2048 tokens of 36 heads (rope_unit), 47 us against 41 us for 6007 tokens of 36 heads (rms_rope).
+// every pair twice, table entries one by one, and divide 64-bit indices per head row: 171 us against 88 us for
+// 8 x 2048 tokens of 36 heads (rope_unit), 165 us against 96 us for the same, 70 against 40 for 6007 tokens (rms_rope).
 // ------------------------------------------------------------------------------------------------
+// The rotation, rounded where the general kernels round it.  Which of the two products of the second side enters its sum
+// rounded is the compiler's choice there, and not the same in both (OWN_ROUNDED: the channel's own); sums of squares
+// run in the general kernels' order too, so that a call gives the same bits on either route.
+template <bool OWN_ROUNDED>
 __device__ __forceinline__ void turn4(float (&x)[4], float (&y)[4], const float (&c)[4], const float (&s)[4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float u = x[e], v = y[e];
-        x[e] = u * c[e] - v * s[e];
-        y[e] = v * c[e] + u * s[e];
+        x[e] = __fmaf_rn(u, c[e], -__fmul_rn(v, s[e]));
+        y[e] = OWN_ROUNDED ? __fmaf_rn(u, s[e], __fmul_rn(v, c[e])) : __fmaf_rn(v, c[e], __fmul_rn(u, s[e]));
     }
 }
 
@@ -266,18 +270,22 @@ __global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUni
         const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + p.Hkv;
         const int h = is_q ? hh : (is_v ? hh - p.Hq - p.Hkv : hh - p.Hq);
         if (__any_sync(0xffffffffu, !is_v)) {  // the other half-warp may hold another kind of row
-            float u[4], v[4], ss = 0.f;
+            float u[4], v[4], su = 0.f, sv = 0.f;
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 u[e] = x[i][e];
                 v[e] = y[i][e];
             }
-            turn4(u, v, c, s);
+            turn4<false>(u, v, c, s);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) ss = fmaf(u[e], u[e], fmaf(v[e], v[e], ss));
+            for (int e = 0; e < 4; ++e) {
+                su = fmaf(u[e], u[e], su);
+                sv = fmaf(v[e], v[e], sv);
+            }
+            float ss = __fadd_rn(su, sv);
 #pragma unroll
             for (int off = 8; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-            float f = rsqrtf(ss * (1.f / 128.f) + p.eps);
+            float f = rsqrtf(__fadd_rn(__fmul_rn(ss, 1.f / 128.f), p.eps));
             if (is_q) f *= p.q_scale;
             if (!is_v) {
 #pragma unroll
@@ -296,31 +304,48 @@ __global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUni
     }
 }
 
-// One CTA per token; a thread holds its NI pieces of q, k and v from the norm's sums to the store.
+// One CTA of 128 threads per token; half-warp g holds heads g, g + 8, ... of q, then of k, then of v (NI pieces in all)
+// from the norm's sums to the store: a thread of the general kernel adds up the same channels of the same heads in one
+// chain.  (256 threads, each half with half of the pieces and its chain going on from the other's: 10 us instead of 12 for
+// 256 rows of 36 heads, 127 instead of 96 for 8 x 2048.)
 template <int NI>
-__global__ void __launch_bounds__(256) rms_rope_append_128_kernel(const RmsRopeParams r) {
+__global__ void __launch_bounds__(128) rms_rope_append_128_kernel(const RmsRopeParams r) {
     const RopeUnitParams &p = r.a;
     __shared__ float s_part[2][8];
-    const int tid = threadIdx.x, j = tid & 15;
+    const int tid = threadIdx.x, j = tid & 15, g = tid >> 4;
     const long long row = blockIdx.x;
     const int b = (int)(blockIdx.x / (unsigned)p.T), t = (int)(blockIdx.x - (unsigned)b * (unsigned)p.T);
-    const int Hk = p.k ? p.Hkv : 0, heads = p.Hq + 2 * Hk;
-    float x[NI][4], y[NI][4], sq = 0.f, sk = 0.f;
+    const int Hk = p.k ? p.Hkv : 0, q_pieces = (p.Hq + 7) / 8, k_pieces = (Hk + 7) / 8;
+    auto place = [&](int i, int &kind, int &h) {  // piece i: kind 0 = q, 1 = k, 2 = v; false past the last head
+        kind = i < q_pieces ? 0 : (i < q_pieces + k_pieces ? 1 : 2);
+        h = g + 8 * (i - (kind == 0 ? 0 : (kind == 1 ? q_pieces : q_pieces + k_pieces)));
+        return h < (kind == 0 ? p.Hq : Hk);
+    };
+    auto widen = [](const uint2 &r, float (&o)[4]) {
+        o[0] = bf16lo(r.x); o[1] = bf16hi(r.x); o[2] = bf16lo(r.y); o[3] = bf16hi(r.y);
+    };
+    uint2 lo[NI], hi[NI];  // as they were read: half the registers of widened ones (8 x 2048 tokens of 36 heads 123 us, so 96)
+    float part[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [q or k][side of the rotation]
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-        const int hh = (tid >> 4) + 16 * i;
-        if (hh >= heads) continue;
-        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + Hk;
-        const int h = is_q ? hh : (is_v ? hh - p.Hq - Hk : hh - p.Hq);
-        const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(is_q ? p.q : (is_v ? p.v : p.k)) +
-                                   row * (is_q ? p.q_stride : (is_v ? p.v_stride : p.k_stride)) + h * 128 + 4 * j;
-        get_v(src, x[i]);
-        get_v(src + 64, y[i]);
-        float ss = 0.f;
+        int kind, h;
+        if (!place(i, kind, h)) continue;
+        const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(kind == 0 ? p.q : (kind == 1 ? p.k : p.v)) +
+                                   row * (kind == 0 ? p.q_stride : (kind == 1 ? p.k_stride : p.v_stride)) + h * 128 + 4 * j;
+        lo[i] = *reinterpret_cast<const uint2 *>(src);
+        hi[i] = *reinterpret_cast<const uint2 *>(src + 64);
+        float x[4], y[4];
+        widen(lo[i], x);
+        widen(hi[i], y);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ss = fmaf(x[i][e], x[i][e], fmaf(y[i][e], y[i][e], ss));
-        if (is_q) sq += ss;
-        else if (!is_v) sk += ss;
+        for (int n = 0; n < 2; ++n)
+            if (kind == n) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    part[n][0] = fmaf(x[e], x[e], part[n][0]);
+                    part[n][1] = fmaf(y[e], y[e], part[n][1]);
+                }
+            }
     }
     const int L = p.seqlens[b], pos = L + t;
     if (L < 0 || pos >= p.T_max || pos >= p.rope_len) {  // uniform over the CTA
@@ -330,14 +355,15 @@ __global__ void __launch_bounds__(256) rms_rope_append_128_kernel(const RmsRopeP
     float c[4], s[4];
     get_v(p.cs + (long long)pos * 128 + 4 * j, c);
     get_v(p.cs + (long long)pos * 128 + 64 + 4 * j, s);
+    float sq = __fadd_rn(part[0][0], part[0][1]), sk = __fadd_rn(part[1][0], part[1][1]);
 #pragma unroll
-    for (int off = 16; off; off >>= 1) {
+    for (int off = 8; off; off >>= 1) {
         sq += __shfl_xor_sync(0xffffffffu, sq, off);
         sk += __shfl_xor_sync(0xffffffffu, sk, off);
     }
-    if ((tid & 31) == 0) {
-        s_part[0][tid >> 5] = sq;
-        s_part[1][tid >> 5] = sk;
+    if (j == 0) {
+        s_part[0][g] = sq;
+        s_part[1][g] = sk;
     }
     __syncthreads();
     sq = sk = 0.f;
@@ -349,32 +375,33 @@ __global__ void __launch_bounds__(256) rms_rope_append_128_kernel(const RmsRopeP
     const float fq = 1.f / sqrtf(sq / (float)(p.Hq * 128) + p.eps), fk = Hk ? 1.f / sqrtf(sk / (float)(Hk * 128) + p.eps) : 0.f;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-        const int hh = (tid >> 4) + 16 * i;
-        if (hh >= heads) continue;
-        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + Hk;
-        const int h = is_q ? hh : (is_v ? hh - p.Hq - Hk : hh - p.Hq);
-        if (!is_v) {
+        int kind, h;
+        if (!place(i, kind, h)) continue;
+        float x[4], y[4];
+        widen(lo[i], x);
+        widen(hi[i], y);
+        if (kind != 2) {
             float w[4], v[4];
-            const float f = is_q ? fq : fk, scale = is_q ? p.q_scale : 1.f;
-            get_v((is_q ? r.q_w : r.k_w) + h * 128 + 4 * j, w);
-            get_v((is_q ? r.q_w : r.k_w) + h * 128 + 64 + 4 * j, v);
+            const float f = kind == 0 ? fq : fk, scale = kind == 0 ? p.q_scale : 1.f;
+            get_v((kind == 0 ? r.q_w : r.k_w) + h * 128 + 4 * j, w);
+            get_v((kind == 0 ? r.q_w : r.k_w) + h * 128 + 64 + 4 * j, v);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                x[i][e] *= f * w[e];
-                y[i][e] *= f * v[e];
+                x[e] *= f * w[e];
+                y[e] *= f * v[e];
             }
-            turn4(x[i], y[i], c, s);
+            turn4<true>(x, y, c, s);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                x[i][e] *= scale;
-                y[i][e] *= scale;
+                x[e] *= scale;
+                y[e] *= scale;
             }
         }
-        __nv_bfloat16 *dst = is_q ? static_cast<__nv_bfloat16 *>(p.q_out) + (row * p.Hq + h) * 128
-                             : is_v ? static_cast<__nv_bfloat16 *>(p.v_cache) + b * p.vcache_bs + pos * p.vcache_ts + h * 128
-                                    : static_cast<__nv_bfloat16 *>(p.k_cache) + b * p.cache_bs + pos * p.cache_ts + h * 128;
-        put_v(dst + 4 * j, x[i]);
-        put_v(dst + 64 + 4 * j, y[i]);
+        __nv_bfloat16 *dst = kind == 0   ? static_cast<__nv_bfloat16 *>(p.q_out) + (row * p.Hq + h) * 128
+                             : kind == 1 ? static_cast<__nv_bfloat16 *>(p.k_cache) + b * p.cache_bs + pos * p.cache_ts + h * 128
+                                         : static_cast<__nv_bfloat16 *>(p.v_cache) + b * p.vcache_bs + pos * p.vcache_ts + h * 128;
+        put_v(dst + 4 * j, x);
+        put_v(dst + 64 + 4 * j, y);
     }
 }
 
@@ -564,13 +591,12 @@ int nckv_rms_rope_append(const void *q, const void *k, const void *v, int64_t q_
     const bool vec = (a & (4 * elem - 1)) == 0 && (((uintptr_t)q_weight | (uintptr_t)k_weight) & 15) == 0 && rot_dims % 8 == 0;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)(B * T);
-    const int pieces = (Hq + (k ? 2 * Hkv : 0) + 15) / 16;  // of a thread, 16 heads at a time
+    const int pieces = (Hq + 7) / 8 + (k ? 2 * ((Hkv + 7) / 8) : 0);  // of a thread
     const bool whole = Dk == 128 && Dv == 128 && Dk_pad == 128 && Dv_pad == 128 && rot_dims == 128 && ((uintptr_t)cos_sin & 15) == 0;
-    if (!f32 && vec && whole && pieces <= 4) {
-        if (pieces == 1) rms_rope_append_128_kernel<1><<<grid, 256, 0, s>>>(r);
-        else if (pieces == 2) rms_rope_append_128_kernel<2><<<grid, 256, 0, s>>>(r);
-        else if (pieces == 3) rms_rope_append_128_kernel<3><<<grid, 256, 0, s>>>(r);
-        else rms_rope_append_128_kernel<4><<<grid, 256, 0, s>>>(r);
+    if (!f32 && vec && whole && pieces <= 8) {
+        const auto kernel = pieces <= 2 ? rms_rope_append_128_kernel<2> : pieces <= 4 ? rms_rope_append_128_kernel<4>
+                            : pieces <= 6 ? rms_rope_append_128_kernel<6> : rms_rope_append_128_kernel<8>;
+        kernel<<<grid, 128, 0, s>>>(r);
     } else if (f32) {
         if (vec) rms_rope_append_kernel<float, 4><<<grid, 256, 0, s>>>(r);
         else rms_rope_append_kernel<float, 1><<<grid, 256, 0, s>>>(r);

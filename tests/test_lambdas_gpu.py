@@ -46,9 +46,12 @@ def test_a_changed_scalar_is_seen(name, change, dtype):
     assert not torch.equal(got[0], before[0]) and not torch.equal(got[1], before[1])
 
 
-@torch.inference_mode()
 def test_a_replayed_step_sees_a_written_scalar():
-    model = model_of(3, 256, 2)
+    replayed_step(model_of(3, 256, 2))
+
+
+@torch.inference_mode()
+def replayed_step(model):
     ids = torch.randint(0, 4096, (2, 5), generator=torch.Generator().manual_seed(3)).to(DEV)
     cache = cache_of(model, 2, 64)
     model.forward(ids, kv_cache=cache)
