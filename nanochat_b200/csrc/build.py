@@ -32,7 +32,15 @@ def _nvcc():
 
 
 def up_to_date():
-    return _newer(OUT, [os.path.join(HERE, s) for s in SOURCES + HEADERS]) and _newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])])
+    return _library_current() and _native_current()
+
+
+def _library_current():
+    return _newer(OUT, [os.path.join(HERE, s) for s in SOURCES + HEADERS])
+
+
+def _native_current():
+    return _newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])])
 
 
 def _newer(built, deps):
@@ -63,29 +71,37 @@ def _compile(cmd, verbose):
 
 
 def build(verbose=False, force=False):
-    """Compile the sources side by side, link them, and move each library into place in one step; several
-    processes may call this at the same time."""
+    """Compile the sources of what is not current side by side, link them, and move each library into place in one
+    step; several processes may call this at the same time."""
     if not force and up_to_date():
         return OUT
     with open(os.path.join(PKG, ".build.lock"), "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         if not force and up_to_date():  # another process has built it meanwhile
             return OUT
-        nvcc = _nvcc()
-        flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
-                 "-Xcompiler", "-fvisibility=hidden"] + (["-Xptxas", "-v"] if verbose else [])
-        with tempfile.TemporaryDirectory(dir=PKG, prefix=".build-") as tmp, ThreadPoolExecutor(max(1, os.cpu_count() or 1)) as pool:
-            objs = [os.path.join(tmp, os.path.splitext(s)[0] + ".o") for s in SOURCES]
-            jobs = [[nvcc] + flags + ["-c", "-o", o, os.path.join(HERE, s)] for s, o in zip(SOURCES, objs)]
-            linked, native = os.path.join(tmp, os.path.basename(OUT)), os.path.join(tmp, os.path.basename(NATIVE))
-            if any(list(pool.map(lambda cmd: _compile(cmd, verbose), jobs))) or \
-                    _compile([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "--shared", "-o", linked] + objs, verbose):
-                raise RuntimeError("nvcc failed building libnckv.so")
-            os.replace(linked, OUT)
-            if _compile(_binding_command(native), verbose):
-                raise RuntimeError("the host compiler failed building _native.so")
-            os.replace(native, NATIVE)
+        with tempfile.TemporaryDirectory(dir=PKG, prefix=".build-") as tmp:
+            if force or not _library_current():
+                _build_library(tmp, verbose)
+            if force or not _native_current():
+                native = os.path.join(tmp, os.path.basename(NATIVE))
+                if _compile(_binding_command(native), verbose):
+                    raise RuntimeError("the host compiler failed building _native.so")
+                os.replace(native, NATIVE)
     return OUT
+
+
+def _build_library(tmp, verbose):
+    nvcc = _nvcc()
+    flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
+             "-Xcompiler", "-fvisibility=hidden"] + (["-Xptxas", "-v"] if verbose else [])
+    objs = [os.path.join(tmp, os.path.splitext(s)[0] + ".o") for s in SOURCES]
+    jobs = [[nvcc] + flags + ["-c", "-o", o, os.path.join(HERE, s)] for s, o in zip(SOURCES, objs)]
+    linked = os.path.join(tmp, os.path.basename(OUT))
+    with ThreadPoolExecutor(max(1, min(len(jobs), os.cpu_count() or 1))) as pool:
+        failed = any(list(pool.map(lambda cmd: _compile(cmd, verbose), jobs)))
+    if failed or _compile([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "--shared", "-o", linked] + objs, verbose):
+        raise RuntimeError("nvcc failed building libnckv.so")
+    os.replace(linked, OUT)
 
 
 if __name__ == "__main__":

@@ -1,0 +1,44 @@
+"""What a build compiles (no compiler runs here)."""
+import os
+
+import pytest
+
+from nanochat_b200.csrc import build as b
+
+
+@pytest.fixture
+def built(monkeypatch, tmp_path):
+    """Both libraries in place and newer than every source; returns the list of commands that a build runs."""
+    commands = []
+
+    def compile_(cmd, verbose):
+        commands.append(cmd)
+        with open(cmd[cmd.index("-o") + 1], "w"):
+            return 0
+    monkeypatch.setattr(b, "PKG", str(tmp_path))
+    monkeypatch.setattr(b, "_compile", compile_)
+    for name, path in (("OUT", tmp_path / "libnckv.so"), ("NATIVE", tmp_path / "_native.so")):
+        path.touch()
+        monkeypatch.setattr(b, name, str(path))
+    return commands
+
+
+def test_nothing_to_do(built):
+    assert b.up_to_date() and b.build() == b.OUT and built == []
+
+
+def test_the_binding_alone(built):
+    os.utime(b.NATIVE, (0, 0))
+    b.build()
+    assert [cmd[cmd.index("-o") + 1].endswith("_native.so") for cmd in built] == [True] and b.up_to_date()
+
+
+def test_the_kernels_alone(built):
+    os.utime(b.OUT, (0, 0))
+    b.build()
+    assert len(built) == len(b.SOURCES) + 1 and not any(b.BINDING in cmd for cmd in built) and b.up_to_date()
+
+
+def test_everything_on_demand(built):
+    b.build(force=True)
+    assert len(built) == len(b.SOURCES) + 2
