@@ -130,9 +130,13 @@ lib = _load()
 try:
     import torch  # noqa: F401  (its libraries first: _native is linked against them)
 
+    from .csrc import build as _build
+    if _build.native_built_for() not in (None, _build.native_wanted()):
+        raise ImportError(f"built for {_build.native_built_for()}, not for {_build.native_wanted()}")
     from . import _native as native  # the most repeated calls without ctypes; None from one of them: take the general path
 except ImportError as e:
-    raise ImportError(f"nanochat_b200/_native.so cannot be loaded ({e}): build it with `python -m nanochat_b200.csrc.build`") from e
+    raise ImportError(f"nanochat_b200/_native.so cannot be loaded ({e}): build it with `python -m nanochat_b200.csrc.build`, "
+                      "with --force where that finds nothing to do") from e
 
 
 def check(fn_name, rc):

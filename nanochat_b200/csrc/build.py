@@ -16,6 +16,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 PKG = os.path.dirname(HERE)
 OUT = os.path.join(PKG, "libnckv.so")
 NATIVE = os.path.join(PKG, "_native.so")
+NATIVE_FOR = NATIVE + ".for"  # beside it: what it was built for
 BINDING = os.path.join(HERE, "binding.cpp")
 SOURCES = ["host.cu", "append.cu", "decode_attn.cu", "prefill_broadcast.cu", "lse_combine.cu",
            "prefill_attn.cu", "p2p_exchange.cu", "glue.cu", "flash_attn_bwd.cu", "host_step.cu",
@@ -40,7 +41,22 @@ def _library_current():
 
 
 def _native_current():
-    return _newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])])
+    return _newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])]) and native_built_for() == native_wanted()
+
+
+def native_wanted():
+    """The torch and interpreter that _native.so has to be built for: it holds their tensors' and objects' layouts."""
+    import torch
+    return f"torch {torch.__version__} abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} {sys.implementation.cache_tag}"
+
+
+def native_built_for():
+    """The same of the _native.so that is there; None where nothing says so."""
+    try:
+        with open(NATIVE_FOR) as f:
+            return f.read()
+    except FileNotFoundError:
+        return None
 
 
 def _newer(built, deps):
@@ -86,7 +102,10 @@ def build(verbose=False, force=False):
                 native = os.path.join(tmp, os.path.basename(NATIVE))
                 if _compile(_binding_command(native), verbose):
                     raise RuntimeError("the host compiler failed building _native.so")
+                with open(native + ".for", "w") as f:
+                    f.write(native_wanted())
                 os.replace(native, NATIVE)
+                os.replace(native + ".for", NATIVE_FOR)
     return OUT
 
 

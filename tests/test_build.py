@@ -1,7 +1,10 @@
 """What a build compiles (no compiler runs here)."""
 import os
+import subprocess
+import sys
 
 import pytest
+import torch
 
 from nanochat_b200.csrc import build as b
 
@@ -20,6 +23,9 @@ def built(monkeypatch, tmp_path):
     for name, path in (("OUT", tmp_path / "libnckv.so"), ("NATIVE", tmp_path / "_native.so")):
         path.touch()
         monkeypatch.setattr(b, name, str(path))
+    monkeypatch.setattr(b, "NATIVE_FOR", b.NATIVE + ".for", raising=False)
+    with open(b.NATIVE_FOR, "w") as f:
+        f.write(b.native_wanted() if hasattr(b, "native_wanted") else "")
     return commands
 
 
@@ -42,3 +48,16 @@ def test_the_kernels_alone(built):
 def test_everything_on_demand(built):
     b.build(force=True)
     assert len(built) == len(b.SOURCES) + 2
+
+
+def test_another_torch_asks_for_another_binding(built, monkeypatch):
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
+    assert not b.up_to_date()
+    b.build()
+    assert len(built) == 1 and b.BINDING in built[0] and b.up_to_date()
+
+
+def test_a_binding_for_another_torch_is_not_loaded():
+    code = ("import torch; torch.__version__ += '.other'\n"
+            "try:\n import nanochat_b200._lib\nexcept ImportError as e:\n assert 'built for' in str(e) and '--force' in str(e); raise SystemExit(7)")
+    assert subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(b.PKG + "/"))).returncode == 7
