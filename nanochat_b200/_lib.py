@@ -127,13 +127,23 @@ def _load():
 
 
 lib = _load()
-try:
-    import torch  # noqa: F401  (its libraries first: _native is linked against them)
+class _NothingNative:
+    """Stands in for the native calls under a torch without CUDA, which has no tensors for them: takes nothing."""
 
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+try:
     from .csrc import build as _build
-    if _build.native_built_for() not in (None, _build.native_wanted()):
+    if _build.native_wanted() is None:
+        native = _NothingNative()
+    elif _build.native_built_for() not in (None, _build.native_wanted()):
         raise ImportError(f"built for {_build.native_built_for()}, not for {_build.native_wanted()}")
-    from . import _native as native  # the most repeated calls without ctypes; None from one of them: take the general path
+    else:
+        # the most repeated calls without ctypes; None from one of them: take the general path.  (torch is imported by
+        # now, and its libraries with it, which _native is linked against)
+        from . import _native as native
 except ImportError as e:
     raise ImportError(f"nanochat_b200/_native.so cannot be loaded ({e}): build it with `python -m nanochat_b200.csrc.build`, "
                       "with --force where that finds nothing to do") from e

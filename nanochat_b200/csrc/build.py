@@ -41,12 +41,18 @@ def _library_current():
 
 
 def _native_current():
-    return _newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])]) and native_built_for() == native_wanted()
+    return native_wanted() is None or (_newer(NATIVE, [BINDING, os.path.join(HERE, HEADERS[-1])]) and native_built_for() == native_wanted())
 
 
 def native_wanted():
-    """The torch and interpreter that _native.so has to be built for: it holds their tensors' and objects' layouts."""
-    import torch
+    """The torch and interpreter that _native.so has to be built for: it holds their tensors' and objects' layouts.
+    None where there is no torch, or one without CUDA, whose tensors no native call takes."""
+    try:
+        import torch
+    except ImportError:
+        return None
+    if torch.version.cuda is None:
+        return None
     return f"torch {torch.__version__} abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)} {sys.implementation.cache_tag}"
 
 
@@ -98,7 +104,7 @@ def build(verbose=False, force=False):
         with tempfile.TemporaryDirectory(dir=PKG, prefix=".build-") as tmp:
             if force or not _library_current():
                 _build_library(tmp, verbose)
-            if force or not _native_current():
+            if native_wanted() is not None and (force or not _native_current()):
                 native = os.path.join(tmp, os.path.basename(NATIVE))
                 if _compile(_binding_command(native), verbose):
                     raise RuntimeError("the host compiler failed building _native.so")

@@ -61,3 +61,18 @@ def test_a_binding_for_another_torch_is_not_loaded():
     code = ("import torch; torch.__version__ += '.other'\n"
             "try:\n import nanochat_b200._lib\nexcept ImportError as e:\n assert 'built for' in str(e) and '--force' in str(e); raise SystemExit(7)")
     assert subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(b.PKG + "/"))).returncode == 7
+
+
+def test_a_torch_without_cuda_needs_no_binding(built, monkeypatch):
+    os.remove(b.NATIVE)
+    monkeypatch.setattr(torch.version, "cuda", None)
+    assert b.up_to_date()
+    b.build(force=True)
+    assert len(built) == len(b.SOURCES) + 1 and not any(b.BINDING in cmd for cmd in built)
+
+
+def test_the_package_imports_under_a_torch_without_cuda():
+    code = ("import sys, torch; torch.version.cuda = None; sys.modules['nanochat_b200._native'] = None\n"
+            "from nanochat_b200 import _lib, ops, gpt\n"
+            "try:\n ops.glue_relu_sq(torch.zeros(8, dtype=torch.bfloat16))\nexcept RuntimeError as e:\n assert 'CUDA' in str(e); raise SystemExit(7)")
+    assert subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(b.PKG + "/"))).returncode == 7
