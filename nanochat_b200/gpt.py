@@ -15,6 +15,7 @@ from dataclasses import dataclass, fields
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import ops
 from .flash_attention import flash_attn
@@ -215,6 +216,9 @@ class Block(nn.Module):
         return x + self.mlp(rms(x))
 
 
+_FORWARD = {cls: cls.forward for cls in (CastLinear, Attention, MLP, Block)}
+
+
 @register("nanochat")
 class GPT(nn.Module):
     """Inference-only GPT with the reference's module tree and forward arithmetic (gpt.py:154-481)."""
@@ -356,11 +360,36 @@ class GPT(nn.Module):
         return self._head(rms(x), logits_at)
 
     def _prompt_can_fuse(self, rows, device):
-        """The fused trunk has a widest row and rounds the lambdas as the eager multiply does for bf16 and fp32 ones on
-        the activations' device; the eager trunk takes the rest."""
+        """The fused trunk has a widest row, rounds the lambdas as the eager multiply does for bf16 and fp32 ones on
+        the activations' device, and calls the layers' products without the modules around them; the eager trunk takes
+        the rest, and whatever runs more than a module's own forward."""
         return rows > 0 and self.config.n_embd <= ops.GLUE_MAX_C and all(
             t.device == device and t.dtype in (torch.bfloat16, torch.float32)
-            for t in (self.resid_lambdas, self.x0_lambdas, self.backout_lambda))
+            for t in (self.resid_lambdas, self.x0_lambdas, self.backout_lambda)) and self._layers_as_written()
+
+    def _layers_as_written(self):
+        """Whether a call of any module in the layers runs the forward of its class above and nothing else: no hooks, no
+        forward of a subclass, none put in its place."""
+        if _has_any_global_hook() or any(cls.forward is not forward for cls, forward in _FORWARD.items()):
+            return False
+        attributes = []  # of ten modules a layer, past Module.__getattr__
+        for block in self.transformer.h:
+            if type(block) is not Block:
+                return False
+            attributes.append(block.__dict__)
+            for part in block.__dict__["_modules"].values():
+                if type(part) not in _FORWARD:
+                    return False
+                attributes.append(part.__dict__)
+                for product in part.__dict__["_modules"].values():
+                    if product is not None:
+                        if type(product) is not CastLinear:
+                            return False
+                        attributes.append(product.__dict__)
+        for own in attributes:
+            if own["_forward_hooks"] or own["_forward_pre_hooks"] or "forward" in own:
+                return False
+        return True
 
     def _head(self, x, logits_at):
         """Soft-capped logits of normed activations (B, T, C), at the given places only if there are any given."""
@@ -401,7 +430,8 @@ class GPT(nn.Module):
             x_sum, x, xn = mix(x, add=pending, x0=x0, resid_lambda=resid[i], x0_lambda=x0l[i], want_sum=(i == backout_at + 1))
             if i == backout_at + 1:
                 x_backout = x_sum
-            attn = block.attn
+            attn, mlp = block._modules["attn"], block._modules["mlp"]._modules  # (past Module.__getattr__, ten times a layer)
+            products = attn._modules
             # one token per row: the row count stays, and with it the check; prompts come in all lengths
             w_qkv = attn.fused_qkv_weight(xn) if self.fused_qkv and T == 1 else None
             if w_qkv is not None:  # one product; q, k, v are column slices of its output (the kernels take the stride)
@@ -411,15 +441,15 @@ class GPT(nn.Module):
                 k = qkv[..., nq:nq + nkv].view(B, 1, attn.n_kv_head, attn.head_dim)
                 v = qkv[..., nq + nkv:].view(B, 1, attn.n_kv_head, attn.head_dim)
             else:
-                q = attn.c_q(xn).view(B, T, attn.n_head, attn.head_dim)
-                k = attn.c_k(xn).view(B, T, attn.n_kv_head, attn.head_dim)
-                v = attn.c_v(xn).view(B, T, attn.n_kv_head, attn.head_dim)
+                q = products["c_q"](xn).view(B, T, attn.n_head, attn.head_dim)
+                k = products["c_k"](xn).view(B, T, attn.n_kv_head, attn.head_dim)
+                v = products["c_v"](xn).view(B, T, attn.n_kv_head, attn.head_dim)
             if str(i) in self.value_embeds:
                 ve = self.value_embeds[str(i)](idx).to(x.dtype)
-                v = ops.glue_ve_gate(v, attn.ve_gate(xn[..., :attn.ve_gate_channels]), ve)
+                v = ops.glue_ve_gate(v, products["ve_gate"](xn[..., :attn.ve_gate_channels]), ve)
             y = kv_attention(q, k, v, rope_tables, self.window_sizes[i], kv_cache, i)
-            _, x, xn = ops.glue_mix_norm(x, add=attn.c_proj(y.view(B, T, C)))
-            pending = block.mlp.c_proj(ops.glue_relu_sq(block.mlp.c_fc(xn)))
+            _, x, xn = ops.glue_mix_norm(x, add=products["c_proj"](y.view(B, T, C)))
+            pending = mlp["c_proj"](ops.glue_relu_sq(mlp["c_fc"](xn)))
         if backout_at == n_layer - 1:  # only a one-layer model: the backout operand is the final sum itself
             x_backout, _, _ = ops.glue_mix_norm(x, add=pending, want_sum=True, want_x=False, want_norm=False)
             _, _, xn = mix(x_backout, x_backout=x_backout, backout_lambda=backout, want_x=False)
