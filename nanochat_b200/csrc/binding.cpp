@@ -160,18 +160,22 @@ std::optional<Three> glue_mix_norm(const Tensor &x, const std::optional<Tensor> 
                     });
 }
 
-// The same with the scalars (those of the mix that is asked for) as elements on the rows' device.
+// The same with the scalars (those of the mix that is asked for) in vectors on the rows' device: element `layer` of the
+// first two, the only one of the third.
 std::optional<Three> glue_mix_norm_at(const Tensor &x, const std::optional<Tensor> &add, const std::optional<Tensor> &x0,
-                                      const std::optional<Tensor> &x_backout, const std::optional<Tensor> &resid_lambda,
-                                      const std::optional<Tensor> &x0_lambda, const std::optional<Tensor> &backout_lambda, bool want_sum,
-                                      bool want_x, bool want_norm, double eps) {
+                                      const std::optional<Tensor> &x_backout, const std::optional<Tensor> &resid_lambdas,
+                                      const std::optional<Tensor> &x0_lambdas, const std::optional<Tensor> &backout_lambda, int64_t layer,
+                                      bool want_sum, bool want_x, bool want_norm, double eps) {
     const void *at[3] = {};
     int f32_mask = 0, i = 0;
-    for (const std::optional<Tensor> *t : {&resid_lambda, &x0_lambda, &backout_lambda}) {
+    for (const std::optional<Tensor> *t : {&resid_lambdas, &x0_lambdas, &backout_lambda}) {
         if (*t) {
+            const int64_t n = (*t)->numel(), e = i < 2 ? layer : 0;
             const bool f32 = (*t)->scalar_type() == at::kFloat;
-            if ((*t)->numel() != 1 || (*t)->device() != x.device() || (!f32 && (*t)->scalar_type() != at::kBFloat16)) return std::nullopt;
-            at[i] = (*t)->data_ptr();
+            if (e < 0 || e >= n || (i == 2 && n != 1) || !(*t)->is_contiguous() || (*t)->device() != x.device() ||
+                (!f32 && (*t)->scalar_type() != at::kBFloat16))
+                return std::nullopt;
+            at[i] = static_cast<const char *>((*t)->data_ptr()) + e * (f32 ? 4 : 2);
             f32_mask |= (int)f32 << i;
         }
         ++i;

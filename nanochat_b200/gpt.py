@@ -401,15 +401,16 @@ class GPT(nn.Module):
         return 15 * torch.tanh(z[..., :self.config.vocab_size].float() / 15)
 
     def _lambdas(self, device):
-        """(mixing op, per-layer scalars for it): one-element views that the kernels read, so that a parameter may be
-        written or replaced between any two passes; numbers where a parameter is on another device.  They round to
-        bf16: the eager multiply converts a 0-dim parameter to the activation dtype before it multiplies (and
-        gpt.py:467 casts the backout lambda explicitly)."""
-        params = [t.detach().reshape(-1) for t in (self.resid_lambdas, self.x0_lambdas, self.backout_lambda)]
+        """(arguments of the mix of layer i, those of the backout).  The kernels read the parameters, which may be written
+        or replaced between any two passes; numbers where a parameter is on another device.  They round to bf16: the
+        eager multiply converts a 0-dim parameter to the activation dtype before it multiplies (and gpt.py:467 casts the
+        backout lambda explicitly)."""
+        params = (self.resid_lambdas, self.x0_lambdas, self.backout_lambda)
         if all(t.device == device for t in params):
-            return ops.glue_mix_norm_at, *((t if t.dtype in (torch.bfloat16, torch.float32) else t.to(torch.bfloat16)).unbind()
-                                           for t in params)
-        return ops.glue_mix_norm, *(t.to(torch.bfloat16).float().tolist() for t in params)
+            r, x, b = ((t if t.dtype in (torch.bfloat16, torch.float32) else t.to(torch.bfloat16)).contiguous() for t in params)
+            return ops.glue_mix_norm_at, lambda i: dict(resid_lambdas=r, x0_lambdas=x, layer=i), dict(backout_lambda=b)
+        r, x, b = (t.detach().to(torch.bfloat16).float().reshape(-1).tolist() for t in params)
+        return ops.glue_mix_norm, lambda i: dict(resid_lambda=r[i], x0_lambda=x[i]), dict(backout_lambda=b[0])
 
     def _trunk_fused(self, idx, x, kv_cache, rope_tables):
         """The layer loop of ``forward`` over a cache with the elementwise glue fused, up to the last norm:
@@ -418,7 +419,7 @@ class GPT(nn.Module):
         one), instead of about a dozen eager launches.  Same matrix products, same roundings."""
         B, T = idx.shape
         C = x.size(-1)
-        mix, resid, x0l, (backout,) = self._lambdas(x.device)
+        mix, layer_scalars, backout = self._lambdas(x.device)
         n_layer = self.config.n_layer
         backout_at = n_layer // 2
         x = x.contiguous()
@@ -427,7 +428,7 @@ class GPT(nn.Module):
         x_backout = None
         for i, block in enumerate(self.transformer.h):
             # the residual stream after layer backout_at is needed later: keep the sum when the add happens
-            x_sum, x, xn = mix(x, add=pending, x0=x0, resid_lambda=resid[i], x0_lambda=x0l[i], want_sum=(i == backout_at + 1))
+            x_sum, x, xn = mix(x, add=pending, x0=x0, want_sum=(i == backout_at + 1), **layer_scalars(i))
             if i == backout_at + 1:
                 x_backout = x_sum
             attn, mlp = block._modules["attn"], block._modules["mlp"]._modules  # (past Module.__getattr__, ten times a layer)
@@ -452,9 +453,9 @@ class GPT(nn.Module):
             pending = mlp["c_proj"](ops.glue_relu_sq(mlp["c_fc"](xn)))
         if backout_at == n_layer - 1:  # only a one-layer model: the backout operand is the final sum itself
             x_backout, _, _ = ops.glue_mix_norm(x, add=pending, want_sum=True, want_x=False, want_norm=False)
-            _, _, xn = mix(x_backout, x_backout=x_backout, backout_lambda=backout, want_x=False)
+            _, _, xn = mix(x_backout, x_backout=x_backout, want_x=False, **backout)
         else:
-            _, _, xn = mix(x, add=pending, x_backout=x_backout, backout_lambda=backout, want_x=False)
+            _, _, xn = mix(x, add=pending, x_backout=x_backout, want_x=False, **backout)
         return xn
 
     @torch.inference_mode()

@@ -699,19 +699,26 @@ def glue_mix_norm(x, add=None, x0=None, x_backout=None, resid_lambda=1.0, x0_lam
                      want_sum, want_x, want_norm, eps)
 
 
-def glue_mix_norm_at(x, add=None, x0=None, x_backout=None, resid_lambda=None, x0_lambda=None, backout_lambda=None,
+def glue_mix_norm_at(x, add=None, x0=None, x_backout=None, resid_lambdas=None, x0_lambdas=None, backout_lambda=None, layer=0,
                      want_sum=False, want_x=True, want_norm=True, eps=RMS_EPS):
-    """``glue_mix_norm`` with its scalars on the rows' device, one fp32 or bf16 element each: the kernel reads them
-    when it runs and rounds them to bf16, as the eager multiply by a parameter does."""
-    done = _lib.native.glue_mix_norm_at(x, add, x0, x_backout, resid_lambda, x0_lambda, backout_lambda, want_sum, want_x, want_norm, eps)
+    """``glue_mix_norm`` with its scalars in fp32 or bf16 vectors on the rows' device: element ``layer`` of the first two,
+    the only one of the third.  The kernel reads them when it runs and rounds them to bf16, as the eager multiply by a
+    parameter does."""
+    done = _lib.native.glue_mix_norm_at(x, add, x0, x_backout, resid_lambdas, x0_lambdas, backout_lambda, layer, want_sum, want_x,
+                                        want_norm, eps)
     if done is not None:
         return done
-    scalars = (resid_lambda, x0_lambda, backout_lambda)
-    for s in scalars:
-        if s is not None and (s.device != x.device or s.numel() != 1 or s.dtype not in (torch.float32, torch.bfloat16)):
-            raise RuntimeError("nckv::glue_mix_norm_at needs scalars of one fp32 or bf16 element each on the rows' device")
-    f32_mask = sum((s is not None and s.dtype == torch.float32) << i for i, s in enumerate(scalars))
-    return _mix_norm("glue_mix_norm_at", x, add, x0, x_backout, (*(_ptr(s) for s in scalars), f32_mask), want_sum, want_x, want_norm, eps)
+    at, f32_mask = [], 0
+    for i, t in enumerate((resid_lambdas, x0_lambdas, backout_lambda)):
+        if t is not None:
+            e = layer if i < 2 else 0
+            if t.device != x.device or not t.is_contiguous() or t.dtype not in (torch.float32, torch.bfloat16) or \
+                    not 0 <= e < t.numel() or (i == 2 and t.numel() != 1):
+                raise RuntimeError("nckv::glue_mix_norm_at needs contiguous fp32 or bf16 scalars on the rows' device, one of them for the "
+                                   f"layer (layer {layer}, got {tuple(t.shape)} {t.dtype} on {t.device})")
+            f32_mask |= (t.dtype == torch.float32) << i
+        at.append(ctypes.c_void_p(t.data_ptr() + e * t.element_size() if t is not None else 0))
+    return _mix_norm("glue_mix_norm_at", x, add, x0, x_backout, (*at, f32_mask), want_sum, want_x, want_norm, eps)
 
 
 def _mix_norm(name, x, add, x0, x_backout, scalars, want_sum, want_x, want_norm, eps):

@@ -72,8 +72,9 @@ def test_scalars_on_the_device_mix_as_numbers_do(monkeypatch, C, dtypes):
     from nanochat_b200 import _lib
     gen = torch.Generator().manual_seed(C)
     x, add, other = (torch.randn(5, C, generator=gen).to(DEV, BF) for _ in range(3))
-    lam = [torch.tensor([0.1, v], device=DEV).to(t)[1] for v, t in zip((1.083, 0.1337, 0.2), dtypes)]
-    num = [float(t.to(BF)) for t in lam]
+    lam = [torch.tensor([0.1, v], device=DEV).to(t) for v, t in zip((1.083, 0.1337, 0.2), dtypes)]
+    lam[2] = lam[2][1:]
+    num = [float(t[-1].to(BF)) for t in lam]
     native = _lib.native
 
     class General:
@@ -81,12 +82,13 @@ def test_scalars_on_the_device_mix_as_numbers_do(monkeypatch, C, dtypes):
             return lambda *a: None
     for module in (native, General()):
         monkeypatch.setattr(_lib, "native", module)
-        got = (*ops.glue_mix_norm_at(x, add=add, x0=other, resid_lambda=lam[0], x0_lambda=lam[1], want_sum=True),
+        got = (*ops.glue_mix_norm_at(x, add=add, x0=other, resid_lambdas=lam[0], x0_lambdas=lam[1], layer=1, want_sum=True),
                *ops.glue_mix_norm_at(x, add=add, x_backout=other, backout_lambda=lam[2]), *ops.glue_mix_norm_at(x, want_x=False))
         want = (*ops.glue_mix_norm(x, add=add, x0=other, resid_lambda=num[0], x0_lambda=num[1], want_sum=True),
                 *ops.glue_mix_norm(x, add=add, x_backout=other, backout_lambda=num[2]), *ops.glue_mix_norm(x, want_x=False))
         assert all((a is None) == (b is None) and (a is None or torch.equal(a, b)) for a, b in zip(got, want))
-        for bad in (dict(resid_lambda=lam[0]), dict(resid_lambda=lam[0].cpu(), x0_lambda=lam[1]),
-                    dict(resid_lambda=lam[0].double(), x0_lambda=lam[1]), dict(resid_lambda=torch.ones(2, device=DEV), x0_lambda=lam[1])):
+        for bad in (dict(resid_lambdas=lam[0]), dict(resid_lambdas=lam[0].cpu(), x0_lambdas=lam[1]),
+                    dict(resid_lambdas=lam[0].double(), x0_lambdas=lam[1]), dict(resid_lambdas=lam[0], x0_lambdas=lam[1], layer=2),
+                    dict(resid_lambdas=lam[0], x0_lambdas=lam[1], layer=-1)):
             with pytest.raises(RuntimeError):
                 ops.glue_mix_norm_at(x, x0=other, **bad)
