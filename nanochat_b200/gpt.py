@@ -223,7 +223,10 @@ _FORWARD = {cls: cls.forward for cls in (CastLinear, Attention, MLP, Block)}
 class GPT(nn.Module):
     """Inference-only GPT with the reference's module tree and forward arithmetic (gpt.py:154-481)."""
 
-    accepts_logits_at = True
+    @property
+    def accepts_logits_at(self):
+        """Whether ``forward`` takes ``logits_at``: this class's does, one that stands in its place need not."""
+        return type(self).forward is _GPT_FORWARD and "forward" not in self.__dict__
 
     def __init__(self, config, pad_vocab_size_to=64, compute_dtype=None):
         super().__init__()
@@ -481,3 +484,6 @@ class GPT(nn.Module):
                 nxt = torch.argmax(logits, dim=-1, keepdim=True)
             ids = torch.cat((ids, nxt), dim=1)
             yield nxt.item()
+
+
+_GPT_FORWARD = GPT.forward
