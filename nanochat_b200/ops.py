@@ -152,6 +152,16 @@ _NS.define("append_rope_norm(Tensor q, Tensor k, Tensor v, Tensor(a!) k_cache, T
            "Tensor cache_seqlens, Tensor cos, Tensor sin, float qk_scale, float eps) -> Tensor")
 
 
+def _token_stride(t):
+    """Distance between the tokens of (B, T, H, D) activations with packed heads, or None.  Tokens that share their
+    elements (expanded ones; a distance of 0 means packed to the library) have none."""
+    T, H, D = t.shape[1:]
+    stride = t.stride(1 if T > 1 else 0)
+    ok = t.stride(3) == 1 and t.stride(2) == D and (T == 1 or t.stride(0) == T * stride) and stride >= H * D and \
+        stride % 8 == 0 and t.data_ptr() % 16 == 0
+    return stride if ok else None
+
+
 def _append_rope_norm(q, k, v, k_cache, v_cache, cache_seqlens, cos, sin, qk_scale, eps, write_slots=None, split=None):
     name = "append_rope_norm"
     _require_cuda(name, q, k, v, k_cache, v_cache, cache_seqlens, cos, sin)
@@ -174,11 +184,7 @@ def _append_rope_norm(q, k, v, k_cache, v_cache, cache_seqlens, cos, sin, qk_sca
     # q, k, v may be column slices of one projection output: packed heads, a common token stride per tensor
     strided = None
     if split is None and write_slots is None and not (q.is_contiguous() and k.is_contiguous() and v.is_contiguous()):
-        def token_stride(t, H):
-            ok = t.stride(3) == 1 and t.stride(2) == D and (T_new == 1 or t.stride(0) == T_new * t.stride(1)) and \
-                t.stride(1 if T_new > 1 else 0) % 8 == 0 and t.data_ptr() % 16 == 0
-            return t.stride(1 if T_new > 1 else 0) if ok else None
-        strided = (token_stride(q, Hq), token_stride(k, Hkv), token_stride(v, Hkv))
+        strided = tuple(_token_stride(t) for t in (q, k, v))
         if None in strided:
             strided = None
     if strided is None:
@@ -770,6 +776,18 @@ def glue_logit_cap(z, cols, cap):
 GLUE_MAX_C = 8192  # widest rows of glue_mix_norm
 
 
+def _row_stride(v):
+    """Distance between the rows of (rows..., H, D) activations with packed heads: 0 if they are packed as well, None if
+    there is no such distance or rows share their elements."""
+    if v.is_contiguous():
+        return 0
+    H, D = v.shape[-2:]
+    lead = [(n, s) for n, s in zip(v.shape[:-2], v.stride()[:-2]) if n > 1]
+    ok = v.stride(-1) == 1 and v.stride(-2) == D and all(lead[i][1] == lead[i + 1][0] * lead[i + 1][1] for i in range(len(lead) - 1)) and \
+        lead and lead[-1][1] >= H * D and lead[-1][1] % 8 == 0 and v.data_ptr() % 16 == 0
+    return lead[-1][1] if ok else None
+
+
 def glue_ve_gate(v, gate_lin, ve):
     """v + 3 * sigmoid(gate_lin)[..., None] * ve in one launch (gpt.py:92-95); v, ve: (..., Hkv, 128),
     gate_lin: (..., Hkv) — the output of the gate's linear layer."""
@@ -781,15 +799,9 @@ def glue_ve_gate(v, gate_lin, ve):
     if gate_lin.numel() != rows * Hkv or ve.numel() != v.numel():
         raise RuntimeError(f"nckv::glue_ve_gate: shapes {tuple(v.shape)} / {tuple(gate_lin.shape)} / {tuple(ve.shape)} do not match")
     # v may be a column slice of a projection output: (rows..., Hkv, D) with packed heads and one row stride
-    row_stride = 0
-    if not v.is_contiguous():
-        lead = [(n, s) for n, s in zip(v.shape[:-2], v.stride()[:-2]) if n > 1]
-        regular = v.stride(-1) == 1 and v.stride(-2) == Dh and all(
-            lead[i][1] == lead[i + 1][0] * lead[i + 1][1] for i in range(len(lead) - 1))
-        if regular and lead and lead[-1][1] % 8 == 0 and v.data_ptr() % 16 == 0:
-            row_stride = lead[-1][1]
-        else:
-            v = v.contiguous()
+    row_stride = _row_stride(v)
+    if row_stride is None:
+        row_stride, v = 0, v.contiguous()
     gate_lin, ve = gate_lin.contiguous(), ve.contiguous()
     out = torch.empty(v.shape, dtype=v.dtype, device=v.device)
     idx = v.device.index
