@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) append_rope_norm_kernel(const AppendParam
     pdl_wait_prior_grids();
     const int j = threadIdx.x & 15;
     const int q_heads = p.q_in ? p.Hq : 0, heads_per_tok = q_heads + 2 * p.Hkv;
-    const unsigned half_warp = (blockIdx.x * 256u + threadIdx.x) >> 4, n_tok = (unsigned)p.B * (unsigned)p.T_new;
+    const unsigned half_warp = half_warp_of(blockIdx.x, threadIdx.x), n_tok = (unsigned)p.B * (unsigned)p.T_new;
     unsigned tok = half_warp / (unsigned)p.per_tok;
     const int first = (int)(half_warp - tok * (unsigned)p.per_tok);
     const bool live = tok < n_tok;
@@ -234,7 +234,7 @@ static int launch_append(AppendParams p, cudaStream_t stream) {
     const bool wide = (long long)p.B * p.T_new * heads_per_tok >= APPEND_WIDE_ROWS;
     p.per_tok = wide ? (heads_per_tok + 3) / 4 : heads_per_tok;
     const long long half_warps = (long long)p.B * p.T_new * p.per_tok;
-    if (half_warps > 0xfffffff0LL) {
+    if (half_warps > HALF_WARPS_MOST) {  // a terabyte of rows and more
         set_error("append: B=%d x T_new=%d tokens are too many for one launch", p.B, p.T_new);
         return NCKV_E_UNSUPPORTED;
     }

@@ -23,6 +23,12 @@ int cuda_fail(cudaError_t e, const char *what);
         if (_e != cudaSuccess) return nckv::cuda_fail(_e, #expr); \
     } while (0)
 
+// This thread's half-warp in a grid of 256-thread CTAs.  32 bits hold the number of one as long as it isn't taken from the
+// number of the thread, which wraps from 2^28 half-warps on.
+constexpr long long HALF_WARPS_MOST = 0xfffffff0LL;
+__host__ __device__ constexpr unsigned half_warp_of(unsigned cta, unsigned thread) { return cta * 16u + (thread >> 4); }
+static_assert(half_warp_of((unsigned)(HALF_WARPS_MOST / 16) - 1, 255) == HALF_WARPS_MOST - 1, "the last half-warp of the largest grid");
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

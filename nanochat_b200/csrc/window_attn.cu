@@ -234,7 +234,7 @@ __device__ __forceinline__ void turn4(float (&x)[4], float (&y)[4], const float 
 template <int NB>
 __global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUnitParams p, int per_tok) {
     const int j = threadIdx.x & 15, heads = p.Hq + 2 * p.Hkv;
-    const unsigned half_warp = (blockIdx.x * 256u + threadIdx.x) >> 4, n_tok = (unsigned)p.B * (unsigned)p.T;
+    const unsigned half_warp = half_warp_of(blockIdx.x, threadIdx.x), n_tok = (unsigned)p.B * (unsigned)p.T;
     unsigned tok = half_warp / (unsigned)per_tok;
     const int first = (int)(half_warp - tok * (unsigned)per_tok);
     bool ok = tok < n_tok;
@@ -536,7 +536,7 @@ int nckv_rope_unit_append(const void *q, const void *k, const void *v, int64_t q
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)blocks;
     const bool whole = Dk == 128 && Dv == 128 && Dk_pad == 128 && Dv_pad == 128 && rot_dims == 128 && ((uintptr_t)cos_sin & 15) == 0;
-    if (!f32 && vec && whole && n <= 0xfffffff0LL) {
+    if (!f32 && vec && whole && n <= HALF_WARPS_MOST) {
         const int heads = Hq + 2 * Hkv;
         const bool wide = n >= 32768;  // the chip is full either way: four rows share a table row and the index arithmetic
         const int per_tok = wide ? (heads + 3) / 4 : heads;
