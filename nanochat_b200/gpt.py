@@ -399,7 +399,7 @@ class GPT(nn.Module):
         if logits_at is not None:
             x = x[:, logits_at]
         z = self.lm_head(x)
-        if self.fused_glue and z.is_cuda and z.dtype == torch.bfloat16:
+        if self.fused_glue and z.is_cuda and z.dtype == torch.bfloat16 and z.is_contiguous() and z.size(-1) >= self.config.vocab_size:
             return ops.glue_logit_cap(z, self.config.vocab_size, 15.0)
         return 15 * torch.tanh(z[..., :self.config.vocab_size].float() / 15)
 

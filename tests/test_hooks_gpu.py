@@ -76,3 +76,13 @@ def test_global_hooks_and_class_forwards_run(monkeypatch):
     monkeypatch.setattr(gpt.MLP, "forward", lambda self, x: (calls.append(1), own(self, x))[1])
     model.forward(ids, kv_cache=cache_of(model, 1, 16))
     assert len(calls) == 2
+
+
+@pytest.mark.parametrize("of_head", [lambda z: z[..., :4000], lambda z: z.transpose(0, 1).contiguous().transpose(0, 1), lambda z: z.float()])
+@pytest.mark.parametrize("T", [1, 9])
+def test_logits_of_another_layout(of_head, T):
+    model = model_of(2, 256, 2)
+    ids = torch.randint(0, 4096, (2, T), generator=torch.Generator().manual_seed(3)).to(DEV)
+    want = of_head(model.forward(ids, kv_cache=cache_of(model, 2, 16)))
+    model.lm_head.register_forward_hook(lambda m, a, out: of_head(out))
+    assert torch.equal(model.forward(ids, kv_cache=cache_of(model, 2, 16)), want)
