@@ -4,7 +4,8 @@
 //
 // Every function here takes the plain case only and returns None for anything else (other dtypes, strides or devices, a
 // missing workspace, sizes that do not fit, a call that the library refused); the caller then takes the general Python
-// path, which decides what is wrong and says so.  Nothing is kept between calls but the table of workspaces, which mirrors the caller's.
+// path, which decides what is wrong and says so.  The interpreter lock is given up once the arguments have been looked at: an
+// allocation or a launch may wait for the device, and other threads run meanwhile.  Nothing is kept between calls but the table of workspaces, which mirrors the caller's.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -85,6 +86,7 @@ std::optional<Tensor> kv_attention(const Tensor &q, const Tensor &k, const Tenso
     const auto on = launch_on(dev, (int)B, (int)Hq, (int)Hkv);
     if (!on) return std::nullopt;
 
+    const pybind11::gil_scoped_release unlocked;
     const c10::cuda::CUDAGuard guard(dev);
     const auto opt = q.options();
     Tensor q_rot = at::empty({B, T, Hq, D}, opt);
@@ -137,6 +139,7 @@ std::optional<Three> mix_norm(const Tensor &x, const std::optional<Tensor> &add,
         if (*t && !row_tensor(**t, x)) return std::nullopt;
     const int64_t C = x.size(-1), rows = x.numel() / C;
     if (rows > INT_MAX || C > INT_MAX) return std::nullopt;
+    const pybind11::gil_scoped_release unlocked;
     const c10::cuda::CUDAGuard guard(x.device());
     Three out;
     auto &[sum, y, norm] = out;
@@ -188,6 +191,7 @@ std::optional<Three> glue_mix_norm_at(const Tensor &x, const std::optional<Tenso
 
 std::optional<Tensor> glue_relu_sq(const Tensor &h) {
     if (!h.is_cuda() || !row_tensor(h, h)) return std::nullopt;
+    const pybind11::gil_scoped_release unlocked;
     const c10::cuda::CUDAGuard guard(h.device());
     Tensor out = at::empty_like(h);
     if (nckv_glue_relu_sq(h.data_ptr(), out.data_ptr(), h.numel(), at::cuda::getCurrentCUDAStream(h.device().index()).stream()) < 0)
