@@ -71,7 +71,7 @@ std::optional<Tensor> kv_attention(const Tensor &q, const Tensor &k, const Tenso
         return std::nullopt;
     const bool paged = block_table.has_value();
     if (paged && (T != 1 || block_table->scalar_type() != at::kInt || block_table->device() != dev || block_table->dim() != 2 ||
-                  block_table->size(0) != B || !block_table->is_contiguous()))
+                  block_table->size(0) != B || !block_table->is_contiguous() || k_cache.size(1) % nckv_paged_tile_tokens()))
         return std::nullopt;
     if (k_cache.sizes() != v_cache.sizes() || k_cache.strides() != v_cache.strides() || (!paged && k_cache.size(0) != B) ||
         k_cache.size(2) != Hkv || k_cache.size(3) != D || k_cache.stride(3) != 1 || k_cache.stride(2) != D)
