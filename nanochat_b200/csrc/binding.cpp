@@ -199,25 +199,12 @@ std::optional<Tensor> glue_relu_sq(const Tensor &h) {
     return out;
 }
 
-// An allocation that finds no memory takes the general path too, whose own raises torch.OutOfMemoryError: as a C++ exception
-// it would reach the caller as a plain RuntimeError, past programs that free memory and try again.
-template <auto Fn> struct OrNone;
-template <typename R, typename... A, R (*Fn)(A...)> struct OrNone<Fn> {
-    static R call(A... a) {
-        try {
-            return Fn(a...);
-        } catch (const c10::OutOfMemoryError &) {
-            return std::nullopt;
-        }
-    }
-};
-
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("set_workspace", &set_workspace);
-    m.def("kv_attention", &OrNone<kv_attention>::call);
-    m.def("glue_mix_norm", &OrNone<glue_mix_norm>::call);
-    m.def("glue_mix_norm_at", &OrNone<glue_mix_norm_at>::call);
-    m.def("glue_relu_sq", &OrNone<glue_relu_sq>::call);
+    m.def("kv_attention", &kv_attention);
+    m.def("glue_mix_norm", &glue_mix_norm);
+    m.def("glue_mix_norm_at", &glue_mix_norm_at);
+    m.def("glue_relu_sq", &glue_relu_sq);
 }
