@@ -12,7 +12,7 @@
 // a token has the same bits however the sequence was cut into calls (see the segments below for the
 // one exception, which is at fp32 rounding level).
 //
-// Mapping.  A CTA owns up to 128 value columns of one (row, head, segment).  A warp owns VG*CL of them (CL = REC_LANE):
+// Mapping.  A CTA owns up to 128 value columns of one (row, head, segment).  A warp owns VG*CL of them (CL: 4 or 8):
 // lane = vg * KG + kg holds key channels {4 KG i + 4 kg + j : i < U, j < 4} of columns {CL vg + c : c < CL}.
 // Pairs of key channels are the two halves of packed fp32 instructions; a step is three of them per
 // pair and column.  Tokens run in batches of 4: their partial outputs are summed over the KG lanes
@@ -66,12 +66,20 @@ struct RecurrentParams {
 
 constexpr int REC_COLS = 128;  // value columns per CTA
 constexpr int REC_TOKENS = 32; // tokens staged at a time, at most
-// Value columns of a lane.  Four: twice the warps of eight for the same columns, which hide each other's latencies (with
-// eight a scheduler had one or two warps and issued in 40 percent of its cycles): per-channel decay, 8 x 2048 tokens, 24
-// heads of 64 x 64, 622 -> 534 us; per-head decay, 1 x 8192, 16 heads of 128 x 128, 560 -> 512.  Eight where a lane has four key
-// channels and a constant decay, which leaves the least work per shared-memory load: 8 x 2048, 12 heads of 64 x 128, 457 us
-// against 463.
-template <int U, bool CHANNEL> constexpr int REC_LANE = !CHANNEL && U == 1 ? 8 : 4;
+// Value columns of a lane, by key channels per lane (4 U) and decay.  us with eight / with four, B200:
+//   constant, 33 to 64 keys, 12 heads of 64 x 128:    8 x 2048 tokens 456 / 462, 64 x 256 327 / 349: eight, the least work per
+//                                                     shared-memory load
+//   constant, 65 to 128 keys, 16 heads of 128 x 128:  1 x 8192 559 / 512, 16 x 1024 766 / 707: four; twice the warps hide each
+//                                                     other's latencies (with eight a scheduler had one or two)
+//   constant, more keys, 8 heads of 256 x 128:        1 x 2048 188 / 190, 8 x 1024 577 / 648: eight (four spills)
+//   per channel, 33 to 64 keys, 24 heads of 64 x 64:  8 x 2048 622 / 534, 64 x 512 860 / 724, 256 x 2 132 / 142: four, but
+//                                                     eight for one batch of tokens of as many rows as below
+//   per channel, 65 to 128, 16 heads of 128 x 128:    1 x 2048 195 / 189, 1 x 8192 645 / 658, 16 x 1024 860 / 945: eight
+//   per channel, more keys, 8 heads of 256 x 128:     1 x 2048 264 / 265, 8 x 1024 964 / 938: four
+//   per channel, up to 32 keys, 24 heads of 32 x 32:  8 x 2048 788 / 491, 32 x 1024 465 / 330, 64 x 512 288 / 322, 64 x 256
+//                                                     149 / 166: four until eight gives the chip eight warps per SM
+template <int U, bool CHANNEL> constexpr int REC_LANE = CHANNEL ? (U == 2 ? 8 : 4) : (U == 2 ? 4 : 8);
+constexpr int REC_WARPS_ENOUGH = 8;  // per SM
 constexpr int REC_BATCH = 4;   // tokens whose outputs are reduced together
 constexpr int REC_MAXQ = 2;    // 4-element pieces a thread stages per vector and chunk
 
@@ -175,9 +183,9 @@ template <int BIT, int LEN> __device__ __forceinline__ int reduce_scatter(float 
 }
 
 // CHANNEL: decay per token and key channel, bonus form.  OUT: false in the first pass over segments.
-template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC>
-__global__ void __launch_bounds__(REC_COLS / (32 * REC_LANE<U, CHANNEL> / KG) * 32) recurrent_kernel(const RecurrentParams p) {
-    constexpr int TB = REC_BATCH, VG = 32 / KG, KP = 4 * KG * U, KQ = KP / 4, CL = REC_LANE<U, CHANNEL>, WC = CL * VG;  // WC: columns per warp
+template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC, int CL>
+__global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kernel(const RecurrentParams p) {
+    constexpr int TB = REC_BATCH, VG = 32 / KG, KP = 4 * KG * U, KQ = KP / 4, WC = CL * VG;  // WC: columns per warp
     constexpr int NB = KQ > 32 ? KQ / 32 : 1;                               // partial bonus sums per token
     const int NT = blockDim.x, NW = NT >> 5;
     const int VP = NW * WC, VQ = VP / 4;
@@ -561,9 +569,9 @@ static cudaError_t rec_step_launch(RecurrentParams p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC>
+template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC, int CL = REC_LANE<U, CHANNEL>>
 static cudaError_t rec_launch_one(RecurrentParams p, cudaStream_t s) {
-    constexpr int TB = REC_BATCH, WC = 32 * REC_LANE<U, CHANNEL> / KG, KP = 4 * KG * U;
+    constexpr int TB = REC_BATCH, WC = 32 * CL / KG, KP = 4 * KG * U;
     const int cols = p.Dv < REC_COLS ? p.Dv : REC_COLS;
     int NW = (cols + WC - 1) / WC;
     while (REC_MAXQ * NW * 32 < TB * (KP / 4)) ++NW;  // room to stage a batch (wide keys, few value columns)
@@ -579,16 +587,22 @@ static cudaError_t rec_launch_one(RecurrentParams p, cudaStream_t s) {
     const size_t smem = sizeof(float) * (2ull * KP + VP + 2ull * C * (KP + VP + (OUT ? KP : 0) + (CHANNEL ? KP : 0) + (OUT && CHANNEL ? 4 : 0)) +
                                          (OUT ? 2ull * C * VP : 0));
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<T, KG, U, CHANNEL, OUT, VEC>,
+        const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<T, KG, U, CHANNEL, OUT, VEC, CL>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    recurrent_kernel<T, KG, U, CHANNEL, OUT, VEC><<<dim3(p.H * p.n_cols, p.B, p.n_seg), NT, smem, s>>>(p);
+    recurrent_kernel<T, KG, U, CHANNEL, OUT, VEC, CL><<<dim3(p.H * p.n_cols, p.B, p.n_seg), NT, smem, s>>>(p);
     return cudaGetLastError();
 }
 
 template <typename T, bool CHANNEL, bool OUT, bool VEC>
 static cudaError_t rec_launch_dims(const RecurrentParams &p, cudaStream_t s) {
+    if constexpr (CHANNEL && OUT) {
+        const int cols = p.Dk <= 32 ? 32 : 16;  // of a warp with eight a lane
+        const bool enough = (long long)p.B * p.H * p.n_seg * ((p.Dv + cols - 1) / cols) >= (long long)REC_WARPS_ENOUGH * sm_count();
+        if (p.Dk <= 32 && enough) return rec_launch_one<T, 8, 1, CHANNEL, OUT, VEC, 8>(p, s);
+        if (p.Dk > 32 && p.Dk <= 64 && p.T <= REC_BATCH && enough) return rec_launch_one<T, 16, 1, CHANNEL, OUT, VEC, 8>(p, s);
+    }
     if (p.Dk <= 32) return rec_launch_one<T, 8, 1, CHANNEL, OUT, VEC>(p, s);
     if (p.Dk <= 64) return rec_launch_one<T, 16, 1, CHANNEL, OUT, VEC>(p, s);
     if (p.Dk <= 128) return rec_launch_one<T, 16, 2, CHANNEL, OUT, VEC>(p, s);
