@@ -177,11 +177,13 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_cap_kernel(const __grid_
                 if (n0 + c >= p.N || row0 >= p.R) break;  // uniform over the warp
                 float v[32];
                 tmem_ld32(acc + (uint32_t)c, v);
+                if (row0 + lane < p.R) {
 #pragma unroll
-                for (int i = 0; i < 32; i += 4)
-                    *reinterpret_cast<float4 *>(turn + lane * 128 + (((i / 4) ^ (lane & 7)) << 4)) =
-                        make_float4(p.cap * tanhf(v[i] / p.cap), p.cap * tanhf(v[i + 1] / p.cap), p.cap * tanhf(v[i + 2] / p.cap),
-                                    p.cap * tanhf(v[i + 3] / p.cap));
+                    for (int i = 0; i < 32; i += 4)
+                        *reinterpret_cast<float4 *>(turn + lane * 128 + (((i / 4) ^ (lane & 7)) << 4)) =
+                            make_float4(p.cap * tanhf(v[i] / p.cap), p.cap * tanhf(v[i + 1] / p.cap), p.cap * tanhf(v[i + 2] / p.cap),
+                                        p.cap * tanhf(v[i + 3] / p.cap));
+                }
                 __syncwarp();
                 const int n = n0 + c + (lane & 7) * 4;
 #pragma unroll
