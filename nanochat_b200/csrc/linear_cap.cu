@@ -13,9 +13,9 @@
 //   warps 2-9   two warps per 32 rows, each with half of the words: accumulator -> cap -> turned in shared memory ->
 //               128 bytes of a row by 8 lanes
 // Tiles run through the rows first: a group of LC_GROUP word tiles stays in L2 while all rows pass.
-// 16384 rows of 1536 by 32768 words: 1522 us where product and pass took 2110 (the product alone 1289); 256 rows 41
-// and 47, 128 rows 40 and 38, which is where the callers' line lies.  A shorter tanh of 25 instructions gave 2 percent
-// at a third less accuracy: not the bound.
+// 16384 rows of 1536 by 32768 words: 1522 us where product and pass took 2110 (the product alone 1289); which sizes pay is the
+// caller's rule (cap_in_product).  Bound: the results' warps, 11 us for the 256 x 256 caps of a tile, beside which 1536
+// channels of products take 7.  A shorter tanh of 25 instructions gave 2 percent at a third less accuracy.
 // Every wait is bounded; one that runs out sets NCKV_ST_TIMEOUT, the roles stop, copies in flight are waited for, both
 // CTAs leave together and tensor memory is freed.
 #include "nckv_common.cuh"

@@ -139,21 +139,37 @@ def softcap(z, cap):
     return z
 
 
-CAP_ROWS = 256  # fewer rows of logits: a product, then a pass over them (128 rows of 32768: 38 us and 40 in one; 256: 47 and 41)
-
-
 def capped_product(a, w, cap):
     """cap * tanh((a @ w^T) / cap) in fp32, a (rows, K) and w (N, K); many bf16 rows in one launch."""
     rows, K = a.shape
-    if a.dtype == w.dtype == torch.bfloat16 and a.is_cuda and w.device == a.device and rows >= CAP_ROWS and K % 8 == 0 and w.size(1) == K and \
-            w.size(0) > 0 and a.is_contiguous() and w.is_contiguous() and (a.data_ptr() | w.data_ptr()) % 16 == 0 and cap > 0:
-        out = torch.empty(rows, w.size(0), dtype=torch.float32, device=a.device)
-        ws = ops.workspace(a.device, 1, 1, 1)
-        idx, stream = _ctx(a)
-        with ops._device_guard(idx):
-            _lib.call("nckv_linear_cap", _ptr(a), _ptr(w), _ptr(out), rows, w.size(0), K, float(cap), _ptr(ws), stream)
-        return out
+    if a.dtype == w.dtype == torch.bfloat16 and a.is_cuda and w.device == a.device and K % 8 == 0 and w.size(1) == K and \
+            a.is_contiguous() and w.is_contiguous() and (a.data_ptr() | w.data_ptr()) % 16 == 0 and cap > 0 and \
+            cap_in_product(rows, w.size(0), K, torch.cuda.get_device_properties(a.device).multi_processor_count):
+        return linear_cap(a, w, cap)
     return softcap(product(a, w, f32_out=True), cap)
+
+
+def cap_in_product(rows, words, channels, sms):
+    """Whether the cap pays inside the product.  A pair of SMs takes about 11 us for the caps of a tile of 256 x 256 whatever
+    the channels; the library's product and the pass behind it take less for short channels, for a single round of tiles and where
+    much of the last round, or of the ragged tiles, is empty.  us, in one launch / in two, B200: 16384 x 32768 x 1536
+    1564 / 2133, 6007 x 32768 x 2048 613 / 968, 1000 x 32768 x 1536 110 / 148, 2048 x 4096 x 1024 37 / 38, and the other
+    way 16384 x 32768 x 256 1210 / 1177, 256 x 16384 x 2048 38 / 36 (one round), 257 x 32768 x 1536 73 / 56 (half
+    filled), 1025 x 16384 x 1536 78 / 73 (70 percent).  No size measured past these lines loses more than 7 percent."""
+    pairs = sms // 2
+    rounds = -(-(-(-rows // 256) * -(-words // 256)) // pairs)
+    return channels >= 1024 and rounds >= 2 and 4 * rows * words >= 3 * rounds * pairs * 256 * 256
+
+
+def linear_cap(a, w, cap):
+    """The product with the cap inside: packed bf16 a (rows, K) and w (N, K), K a multiple of 8."""
+    rows, K = a.shape
+    out = torch.empty(rows, w.size(0), dtype=torch.float32, device=a.device)
+    ws = ops.workspace(a.device, 1, 1, 1)
+    idx, stream = _ctx(a)
+    with ops._device_guard(idx):
+        _lib.call("nckv_linear_cap", _ptr(a), _ptr(w), _ptr(out), rows, w.size(0), K, float(cap), _ptr(ws), stream)
+    return out
 
 
 def rope_unit_append(q, k, v, cos_sin, rot_dims, k_cache, v_cache, cache_seqlens, B, T, heads, kv_heads, dim, vdim,
