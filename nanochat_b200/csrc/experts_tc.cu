@@ -7,10 +7,13 @@
 //   warp 0      moves the weights, and without UP the positions (rows of act), by TMA
 //   warps 6-13  UP: the tokens of a tile lie anywhere in h; these warps fetch them with 16-byte asynchronous copies
 //               into the place the swizzle gives them, so h is never copied into sorted order (a gather by
-//               TMA, four rows per instruction, was three times slower than the products).  With four stages four
-//               groups of two warps take a step each in turn; a group waits for its own copies, so four steps
-//               are on their way at any time (two groups that handed a step over behind the next one's request
-//               had two: 178 us at 6007 tokens x 4 of 16 experts of 1536 x 1024, now 154).
+//               TMA, four rows per instruction, was three times slower than the products).  A group of warps takes a
+//               step at a time and waits for its own copies.  With four stages (wide tiles) four groups of two: four
+//               steps are on their way at any time (two groups that handed a step over behind the next one's request
+//               had two: 178 us at 6007 tokens x 4 of 16 experts of 1536 x 1024, now 154).  With six stages (narrow
+//               tiles) two groups of four, two steps on their way: handed over two of its own steps later, which has
+//               six, a step took longer: 25.6 against 29.0 us at 32 tokens, 41.5 / 43.7 at 512, 60.5 / 66.3 at 1024,
+//               104 / 112 at 2300.
 //   warp 1      one thread issues the products into one of two accumulators
 //   warps 2-5   one thread per position reads the other accumulator, applies the router's weight and the
 //               activation (UP) or finds the pair's place (down); results are turned in shared memory and stored 128

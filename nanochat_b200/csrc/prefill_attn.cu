@@ -352,7 +352,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         uint32_t n_o0 = 0, n_o1 = 0;  // phases of bar_o[0] / bar_o[1] used up by the items before this one
         // All lanes ask once, which is one instruction; only when that fails one lane polls (32 lanes polling one mbarrier are
         // served one after the other) and the warp follows.  With a poll by one lane from the start, its branches and
-        // the shuffle stood in every tile: 8 x 2048 tokens, 12 heads 117 us, now 112.
+        // the shuffle stand in every tile: 8 x 2048 tokens, 12 heads, one / all, timed in turn as the GPU got hotter: 117 / 111,
+        // 117 / 117, 123 / 120, 120 / 115 us.
         auto warp_wait = [&](uint64_t *bar, uint32_t parity) -> bool {
             if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
             int ok = *abort_flag == 0;

@@ -6,11 +6,10 @@
 namespace nckv {
 
 // True in one thread of a converged warp.  The roles that issue products or copies are entered through it and not
-// through a comparison with the lane's number: only then does the compiler know that one thread runs what follows, and
-// keeps descriptors and addresses of tcgen05 and TMA instructions in uniform registers (otherwise each such
-// instruction gets a loop over the active lanes around it).  Attention of 8 x 2048 tokens, 12 heads, whose issuing
-// thread was busy for the whole of a tile: forward 124 -> 111 us, dQ 216 -> 180, dK / dV 269 -> 258; the experts'
-// first product of 6007 tokens 178 -> 170 us.
+// through a comparison with the lane's number, behind which issuing is slower: by clock stamps 400 cycles for 4 P V
+// products and 900 for 8 score products of attention, whose issuing thread was busy for the whole of a tile.  (Presumably
+// the compiler can only then tell that a single thread runs what follows.)  Attention of 8 x 2048 tokens, 12 heads:
+// forward 124 -> 111 us, dQ 216 -> 180, dK / dV 269 -> 258; the experts' first product of 6007 tokens 178 -> 170 us.
 __device__ __forceinline__ bool elect_one() {
     uint32_t one;
     asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.b32 %0, 1, 0, p;\n}" : "=r"(one));
