@@ -225,8 +225,9 @@ static int check_common(const void *k_in, const void *v_in, void *k_cache, void 
 
 // Rows per half-warp.  Few rows (a decode step): one each, the shortest chain from the input to the store.  From
 // APPEND_WIDE_ROWS head rows on the chip is full either way, and four rows share the index arithmetic and the
-// token's table row: 3 x 1531 tokens of 24 head rows take 17 us (56 MB), against 37 us for one row per half-warp
-// with the two sides of a rotation pair in different lanes.
+// token's table row.  us with one / with four: 1536 head rows 7.2 / 9.2, 16800 10.8 / 11.2, 24000 11.2 / 11.2, 33600 13.3 /
+// 13.2, 49152 17 / 15.4, 110232 27.6 / 23.5, 589824 108.5 / 84.5 (one row each with the two sides of a rotation pair in different
+// lanes: 9.2, 13.2, 16.8, 19.4, 23.5, 42, 188).
 constexpr long long APPEND_WIDE_ROWS = 32768;
 
 static int launch_append(AppendParams p, cudaStream_t stream) {

@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(256) rms_rope_append_kernel(const RmsRopeParam
 // ------------------------------------------------------------------------------------------------
 // Both appends for heads of 128 channels that are rotated as a whole, in bf16: lane j of a half-warp holds channels
 // 4j .. 4j + 3 and 64 + 4j .. 64 + 4j + 3 of a head, the two sides of its rotation pairs.  The general kernels load
-// every pair twice, table entries one by one, and divide 64-bit indices per head row: 171 us against 88 us for
-// 8 x 2048 tokens of 36 heads (rope_unit), 165 us against 96 us for the same, 70 against 40 for 6007 tokens (rms_rope).
+// every pair twice, table entries one by one, and divide 64-bit indices per head row: 171 us against 78 us for
+// 8 x 2048 tokens of 36 heads (rope_unit), 166 us against 95 us for the same, 70 against 40 for 6007 tokens (rms_rope).
 // ------------------------------------------------------------------------------------------------
 // The rotation, rounded where the general kernels round it.  Which of the two products of the second side enters its sum
 // rounded is the compiler's choice there, and not the same in both (OWN_ROUNDED: the channel's own); sums of squares
@@ -230,29 +230,24 @@ __device__ __forceinline__ void turn4(float (&x)[4], float (&y)[4], const float 
     }
 }
 
-// NB head rows of one token per half-warp: rows first, first + per_tok, ...
-template <int NB>
-__global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUnitParams p, int per_tok) {
+// One head row per half-warp.  (Four of one token, which share its table row and the index arithmetic, were slower from 36000 head
+// rows on: 8 x 2048 tokens of 36 heads 87 us against 78, 64 x 512 of 24 heads 111 / 100, 2048 of 24 heads 15.4 / 13.3.)
+__global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUnitParams p) {
     const int j = threadIdx.x & 15, heads = p.Hq + 2 * p.Hkv;
     const unsigned half_warp = half_warp_of(blockIdx.x, threadIdx.x), n_tok = (unsigned)p.B * (unsigned)p.T;
-    unsigned tok = half_warp / (unsigned)per_tok;
-    const int first = (int)(half_warp - tok * (unsigned)per_tok);
+    unsigned tok = half_warp / (unsigned)heads;
+    const int hh = (int)(half_warp - tok * (unsigned)heads);
     bool ok = tok < n_tok;
     if (!ok) tok = n_tok - 1;  // stays for the shuffles
     const int b = (int)(tok / (unsigned)p.T), t = (int)(tok - (unsigned)b * (unsigned)p.T);
-    float x[NB][4], y[NB][4];
-#pragma unroll
-    for (int i = 0; i < NB; ++i) {
-        const int hh = first + i * per_tok;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[i][e] = y[i][e] = 0.f;
-        if (!ok || hh >= heads) continue;
-        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + p.Hkv;
-        const int h = is_q ? hh : (is_v ? hh - p.Hq - p.Hkv : hh - p.Hq);
+    const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + p.Hkv;
+    const int h = is_q ? hh : (is_v ? hh - p.Hq - p.Hkv : hh - p.Hq);
+    float x[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+    if (ok) {
         const __nv_bfloat16 *src = static_cast<const __nv_bfloat16 *>(is_q ? p.q : (is_v ? p.v : p.k)) +
                                    tok * (is_q ? p.q_stride : (is_v ? p.v_stride : p.k_stride)) + h * 128 + 4 * j;
-        get_v(src, x[i]);
-        get_v(src + 64, y[i]);
+        get_v(src, x);
+        get_v(src + 64, y);
     }
     const int L = p.seqlens[b], pos = L + t;
     if (ok && (L < 0 || pos >= p.T_max || pos >= p.rope_len)) {
@@ -264,44 +259,38 @@ __global__ void __launch_bounds__(256) rope_unit_append_128_kernel(const RopeUni
         get_v(p.cs + (long long)pos * 128 + 4 * j, c);
         get_v(p.cs + (long long)pos * 128 + 64 + 4 * j, s);
     }
+    if (__any_sync(0xffffffffu, !is_v)) {  // the other half-warp may hold another kind of row
+        float u[4], v[4], su = 0.f, sv = 0.f;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-        const int hh = first + i * per_tok;
-        const bool is_q = hh < p.Hq, is_v = hh >= p.Hq + p.Hkv;
-        const int h = is_q ? hh : (is_v ? hh - p.Hq - p.Hkv : hh - p.Hq);
-        if (__any_sync(0xffffffffu, !is_v)) {  // the other half-warp may hold another kind of row
-            float u[4], v[4], su = 0.f, sv = 0.f;
+        for (int e = 0; e < 4; ++e) {
+            u[e] = x[e];
+            v[e] = y[e];
+        }
+        turn4<false>(u, v, c, s);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            su = fmaf(u[e], u[e], su);
+            sv = fmaf(v[e], v[e], sv);
+        }
+        float ss = __fadd_rn(su, sv);
+#pragma unroll
+        for (int off = 8; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+        float f = rsqrtf(__fadd_rn(__fmul_rn(ss, 1.f / 128.f), p.eps));
+        if (is_q) f *= p.q_scale;
+        if (!is_v) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                u[e] = x[i][e];
-                v[e] = y[i][e];
-            }
-            turn4<false>(u, v, c, s);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                su = fmaf(u[e], u[e], su);
-                sv = fmaf(v[e], v[e], sv);
-            }
-            float ss = __fadd_rn(su, sv);
-#pragma unroll
-            for (int off = 8; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-            float f = rsqrtf(__fadd_rn(__fmul_rn(ss, 1.f / 128.f), p.eps));
-            if (is_q) f *= p.q_scale;
-            if (!is_v) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    x[i][e] = u[e] * f;
-                    y[i][e] = v[e] * f;
-                }
+                x[e] = u[e] * f;
+                y[e] = v[e] * f;
             }
         }
-        if (!ok || hh >= heads) continue;
-        __nv_bfloat16 *dst = is_q ? static_cast<__nv_bfloat16 *>(p.q_out) + ((long long)tok * p.Hq + h) * 128
-                             : is_v ? static_cast<__nv_bfloat16 *>(p.v_cache) + b * p.vcache_bs + pos * p.vcache_ts + h * 128
-                                    : static_cast<__nv_bfloat16 *>(p.k_cache) + b * p.cache_bs + pos * p.cache_ts + h * 128;
-        put_v(dst + 4 * j, x[i]);
-        put_v(dst + 64 + 4 * j, y[i]);
     }
+    if (!ok) return;
+    __nv_bfloat16 *dst = is_q ? static_cast<__nv_bfloat16 *>(p.q_out) + ((long long)tok * p.Hq + h) * 128
+                         : is_v ? static_cast<__nv_bfloat16 *>(p.v_cache) + b * p.vcache_bs + pos * p.vcache_ts + h * 128
+                                : static_cast<__nv_bfloat16 *>(p.k_cache) + b * p.cache_bs + pos * p.cache_ts + h * 128;
+    put_v(dst + 4 * j, x);
+    put_v(dst + 64 + 4 * j, y);
 }
 
 // One CTA of 128 threads per token; half-warp g holds heads g, g + 8, ... of q, then of k, then of v (NI pieces in all)
@@ -537,12 +526,7 @@ int nckv_rope_unit_append(const void *q, const void *k, const void *v, int64_t q
     const unsigned grid = (unsigned)blocks;
     const bool whole = Dk == 128 && Dv == 128 && Dk_pad == 128 && Dv_pad == 128 && rot_dims == 128 && ((uintptr_t)cos_sin & 15) == 0;
     if (!f32 && vec && whole && n <= HALF_WARPS_MOST) {
-        const int heads = Hq + 2 * Hkv;
-        const bool wide = n >= 32768;  // the chip is full either way: four rows share a table row and the index arithmetic
-        const int per_tok = wide ? (heads + 3) / 4 : heads;
-        const unsigned ctas = (unsigned)(((long long)B * T * per_tok + 15) / 16);
-        if (wide) rope_unit_append_128_kernel<4><<<ctas, 256, 0, s>>>(p, per_tok);
-        else rope_unit_append_128_kernel<1><<<ctas, 256, 0, s>>>(p, per_tok);
+        rope_unit_append_128_kernel<<<(unsigned)((n + 15) / 16), 256, 0, s>>>(p);
     } else if (f32) {
         if (vec) rope_unit_append_kernel<float, 4><<<grid, 256, 0, s>>>(p);
         else rope_unit_append_kernel<float, 1><<<grid, 256, 0, s>>>(p);
