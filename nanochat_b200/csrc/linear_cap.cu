@@ -13,9 +13,10 @@
 //   warps 2-9   two warps per 32 rows, each with half of the words: accumulator -> cap -> turned in shared memory ->
 //               128 bytes of a row by 8 lanes
 // Tiles run through the rows first: a group of LC_GROUP word tiles stays in L2 while all rows pass.
-// 16384 rows of 1536 by 32768 words: 1522 us where product and pass took 2110 (the product alone 1289); which sizes pay is the
-// caller's rule (cap_in_product).  Bound: the results' warps, 11 us for the 256 x 256 caps of a tile, beside which 1536
-// channels of products take 7.  A shorter tanh of 25 instructions gave 2 percent at a third less accuracy.
+// 16384 rows of 1536 by 32768 words: 1302 us where product and pass take 1957 (the product alone 1289); which sizes pay is the
+// caller's rule (cap_in_product).  Bound: the tensor pipe (80 percent of its cycles busy, by ncu) under the power limit; the caps of a tile
+// take 7.6 us beside it.  With a division for each value they took 11 and were the bound (1526 us; 4096 rows 373, now 299; 2048 rows
+// of 2048 226, now 186; 1000 rows 120, now 101).  A shorter tanh gave 2 percent at a third less accuracy.
 // Every wait is bounded; one that runs out sets NCKV_ST_TIMEOUT, the roles stop, copies in flight are waited for, both
 // CTAs leave together and tensor memory is freed.
 #include "nckv_common.cuh"
@@ -37,6 +38,30 @@ struct LinearCapParams {
     int R, N, K;
 };
 
+// v / cap for two values, correctly rounded (to the bits of the division) where quotient and residue are normal numbers: the product with
+// the rounded reciprocal, corrected twice by its exact residue (Markstein's method; a uniform divisor leaves 2.5 instructions a value where
+// a division takes about ten and a check).  Values beyond 16 caps count as 16 caps, whose tanh is 1 too, so that an infinite one
+// leaves a quotient; what is no number stays none.
+struct CapQuotient {
+    float2 neg_cap, rcp;
+    float most;
+    __device__ __forceinline__ explicit CapQuotient(float cap)
+        : neg_cap(make_float2(-cap, -cap)), rcp(make_float2(1.f / cap, 1.f / cap)), most(16.f * cap) {}
+    __device__ __forceinline__ float within(float v) const {  // |most| > 0: the sign is v's
+        float r;
+        asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(most));
+        return r;
+    }
+    __device__ __forceinline__ float2 operator()(float v0, float v1) const {
+        const float2 v = make_float2(within(v0), within(v1));
+        float2 q = fmul2(v, rcp);
+        q = ffma2(ffma2(neg_cap, q, v), rcp, q);
+        return ffma2(ffma2(neg_cap, q, v), rcp, q);
+    }
+};
+
+// QUOTIENT: the cap is far from the ends of the numbers, where its reciprocal and the residues are exact enough; else plain divisions.
+template <bool QUOTIENT>
 __global__ void __launch_bounds__(LC_THREADS, 1) linear_cap_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                                                                    const LinearCapParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -154,6 +179,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_cap_kernel(const __grid_
         const int q = warp & 3, part = (warp - 2) >> 2;  // a warp reaches tensor-memory lanes 32 (warp % 4) ..
         uint8_t *turn = smem + LC_STAGES * LC_STAGE + (warp - 2) * LC_TURN;
         const bool vec = p.N % 4 == 0;
+        const CapQuotient quotient(p.cap);
         auto warp_wait = [&](uint64_t *bar, uint32_t parity) -> bool {
             if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
             int ok = 1;
@@ -179,10 +205,12 @@ __global__ void __launch_bounds__(LC_THREADS, 1) linear_cap_kernel(const __grid_
                 tmem_ld32(acc + (uint32_t)c, v);
                 if (row0 + lane < p.R) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4)
+                    for (int i = 0; i < 32; i += 4) {
+                        const float2 x = QUOTIENT ? quotient(v[i], v[i + 1]) : make_float2(v[i] / p.cap, v[i + 1] / p.cap);
+                        const float2 y = QUOTIENT ? quotient(v[i + 2], v[i + 3]) : make_float2(v[i + 2] / p.cap, v[i + 3] / p.cap);
                         *reinterpret_cast<float4 *>(turn + lane * 128 + (((i / 4) ^ (lane & 7)) << 4)) =
-                            make_float4(p.cap * tanhf(v[i] / p.cap), p.cap * tanhf(v[i + 1] / p.cap), p.cap * tanhf(v[i + 2] / p.cap),
-                                        p.cap * tanhf(v[i + 3] / p.cap));
+                            make_float4(p.cap * tanhf(x.x), p.cap * tanhf(x.y), p.cap * tanhf(y.x), p.cap * tanhf(y.y));
+                    }
                 }
                 __syncwarp();
                 const int n = n0 + c + (lane & 7) * 4;
@@ -247,7 +275,8 @@ extern "C" int nckv_linear_cap(const void *x, const void *w, float *out, int R, 
     LinearCapParams p;
     p.out = out; p.status = status; p.cap = cap;
     p.R = R; p.N = N; p.K = K;
-    NCKV_CUDA_CHECK(cudaFuncSetAttribute(linear_cap_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM));
+    const auto kernel = cap >= 0x1p-60f && cap <= 0x1p60f ? linear_cap_kernel<true> : linear_cap_kernel<false>;
+    NCKV_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM));
     const int most = sm_count() / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * (tiles < most ? (int)tiles : most)));
@@ -261,6 +290,6 @@ extern "C" int nckv_linear_cap(const void *x, const void *w, float *out, int R, 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    NCKV_CUDA_CHECK(cudaLaunchKernelEx(&cfg, linear_cap_kernel, mx, mw, p));
+    NCKV_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, mx, mw, p));
     return NCKV_OK;
 }

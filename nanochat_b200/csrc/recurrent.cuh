@@ -153,15 +153,6 @@ template <bool VEC> __device__ __forceinline__ void store_quad(__nv_bfloat16 *p,
     }
 }
 
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-    float2 d;
-    asm("{\n.reg .b64 ra, rb, rd;\nmov.b64 ra, {%2, %3};\nmov.b64 rb, {%4, %5};\nmul.rn.f32x2 rd, ra, rb;\n"
-        "mov.b64 {%0, %1}, rd;\n}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-
 // Sums of o[0 .. LEN) over the lanes that differ in the bits BIT, BIT / 2, .. 1 of `kg`: each level halves
 // what a lane still holds (a single element is summed by both).  Returns the index of the first element left.
 template <int BIT, int LEN> __device__ __forceinline__ int reduce_scatter(float *o, int kg) {

@@ -150,12 +150,12 @@ def capped_product(a, w, cap):
 
 
 def cap_in_product(rows, words, channels, sms):
-    """Whether the cap pays inside the product.  A pair of SMs takes about 11 us for the caps of a tile of 256 x 256 whatever
-    the channels; the library's product and the pass behind it take less for short channels, for a single round of tiles and where
-    much of the last round, or of the ragged tiles, is empty.  us, in one launch / in two, B200: 16384 x 32768 x 1536
-    1564 / 2133, 6007 x 32768 x 2048 613 / 968, 1000 x 32768 x 1536 110 / 148, 2048 x 4096 x 1024 37 / 38, and the other
-    way 16384 x 32768 x 256 1210 / 1177, 256 x 16384 x 2048 38 / 36 (one round), 257 x 32768 x 1536 73 / 56 (half
-    filled), 1025 x 16384 x 1536 78 / 73 (70 percent).  No size measured past these lines loses more than 7 percent."""
+    """Whether the cap pays inside the product.  The library's product and the pass behind it take less where much of the last
+    round of tiles of 256 x 256, or of the ragged tiles, is empty.  us, in one launch / in two, B200: 16384 x 32768 x 1536
+    1294 / 1957, 6007 x 32768 x 2048 580 / 857, 1000 x 32768 x 1536 87 / 147, 2048 x 4096 x 1024 31 / 40, and the other
+    way 257 x 32768 x 1536 55 / 52 (half filled), 300 x 8192 x 1536 25 / 24 (one round, half filled).  Shorter channels (16384 x
+    32768 x 256 853 / 1330), single rounds (256 x 16384 x 2048 34 / 36) and 70 percent (1025 x 16384 x 1536 62 / 73) pay as well by
+    now; the lines lie where they did, for no model here has such heads."""
     pairs = sms // 2
     rounds = -(-(-(-rows // 256) * -(-words // 256)) // pairs)
     return channels >= 1024 and rounds >= 2 and 4 * rows * words >= 3 * rounds * pairs * 256 * 256
