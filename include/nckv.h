@@ -445,7 +445,8 @@ NCKV_API int nckv_glue_ve_gate(const void *v, int64_t v_row_stride, const void *
  * nckv_route: per row the `top` largest of E logits; (row, choice) pairs sorted by expert: slot[i] = row * top +
  *   choice, scale[i] = sigmoid(logit), expert e at [offsets[e], offsets[e + 1]).
  * nckv_experts: up: out[i] = silu(s g) * (s u), [g; u] = w[e] a[slot[i] / top], s = scale[i], w (E, 2 N, K);
- *   else out[slot[i]] = w[e] a[i], w (E, N, K).  R = rows * top pairs.
+ *   else out[slot[i]] = w[e] a[i], w (E, N, K).  R = rows * top pairs.  nckv_experts_scratch: the same with
+ *   nckv_experts_workspace_bytes() of scratch (0: none), 16-byte aligned, with which the up product of many rows is faster.
  */
 NCKV_API int nckv_prefill_attn_split_p(const void *q, const void *k, const void *v, const int32_t *cache_seqlens, void *out,
                       int B, int T_new, int Hq, int Hkv, int D, int T_k, int64_t kv_batch_stride,
@@ -513,6 +514,10 @@ NCKV_API int nckv_route(const float *logits, int32_t *offsets, int32_t *slot, fl
                       void *workspace, size_t workspace_bytes, void *stream);
 NCKV_API int nckv_experts(const void *a, const void *w, void *out, const int32_t *offsets, const int32_t *slot, const float *scale,
                       int up, int R, int E, int top, int N, int K, int f32, int32_t *status, void *stream);
+NCKV_API size_t nckv_experts_workspace_bytes(int up, int R, int E, int N, int K, int f32);
+NCKV_API int nckv_experts_scratch(const void *a, const void *w, void *out, const int32_t *offsets, const int32_t *slot, const float *scale,
+                      int up, int R, int E, int top, int N, int K, int f32, void *workspace, size_t workspace_bytes, int32_t *status,
+                      void *stream);
 
 #ifdef __cplusplus
 }

@@ -96,6 +96,8 @@ SIGNATURES = {
     "nckv_route_workspace_bytes": (c_size_t, [c_int] * 3),
     "nckv_route": (c_int, [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_size_t, c_void_p]),
     "nckv_experts": (c_int, [c_void_p] * 6 + [c_int] * 7 + [c_void_p, c_void_p]),
+    "nckv_experts_workspace_bytes": (c_size_t, [c_int] * 6),
+    "nckv_experts_scratch": (c_int, [c_void_p] * 6 + [c_int] * 7 + [c_void_p, c_size_t, c_void_p, c_void_p]),
 }
 
 ERROR_NAMES = {-1: "NCKV_E_ARG", -2: "NCKV_E_UNSUPPORTED", -3: "NCKV_E_CAPACITY", -4: "NCKV_E_CUDA"}

@@ -421,8 +421,19 @@ int nckv_route(const float *logits, int32_t *offsets, int32_t *slot, float *scal
     return NCKV_OK;
 }
 
+size_t nckv_experts_workspace_bytes(int up, int R, int E, int N, int K, int f32) {
+    using namespace nckv;
+    if (!up || f32 || R <= EXPERT_MANY || E <= 0 || N <= 0 || K <= 0 || K % 8) return 0;
+    return experts_in_pairs(true, R, E, N, K) ? sizeof(__nv_bfloat16) * (size_t)R * K : 0;
+}
+
 int nckv_experts(const void *a, const void *w, void *out, const int32_t *offsets, const int32_t *slot, const float *scale, int up,
                  int R, int E, int top, int N, int K, int f32, int32_t *status, void *stream) {
+    return nckv_experts_scratch(a, w, out, offsets, slot, scale, up, R, E, top, N, K, f32, nullptr, 0, status, stream);
+}
+
+int nckv_experts_scratch(const void *a, const void *w, void *out, const int32_t *offsets, const int32_t *slot, const float *scale, int up,
+                         int R, int E, int top, int N, int K, int f32, void *workspace, size_t workspace_bytes, int32_t *status, void *stream) {
     using namespace nckv;
     if (!a || !w || !out || !offsets || !slot || !status || (up && !scale)) {
         set_error("experts: null pointer argument");
@@ -446,7 +457,9 @@ int nckv_experts(const void *a, const void *w, void *out, const int32_t *offsets
     }
     if (R > EXPERT_MANY) {
         int rc = NCKV_OK;
-        NCKV_CUDA_CHECK(experts_tc(p, up, s, &rc));
+        const bool room = !up || (workspace && !((uintptr_t)workspace & 15) && workspace_bytes >= sizeof(__nv_bfloat16) * (size_t)R * K);
+        if (room && experts_in_pairs(up, R, E, N, K)) NCKV_CUDA_CHECK(experts_pair(p, up, workspace, s, &rc));
+        else NCKV_CUDA_CHECK(experts_tc(p, up, s, &rc));
         return rc;
     }
     if (up) expert_rows_kernel<true><<<dim3((N + 7) / 8, E), ER_WARPS * 32, 0, s>>>(p);

@@ -21,6 +21,11 @@ struct ExpertParams {
     int R, E, top, N, K;
 };
 
+constexpr int EQ_MAX_EXPERTS = 256;
+long long experts_tc_waves(bool up, int R, int E, int N, int bn);  // of tiles of bn weight rows, at an even spread of the positions
+bool experts_tc_wide(bool up, int R, int E, int N);                // whether experts_tc takes the wide ones
+bool experts_in_pairs(bool up, int R, int E, int N, int K);  // whether that many rows take the form on pairs of CTAs
+cudaError_t experts_pair(ExpertParams p, bool up, void *sorted, cudaStream_t s, int *rc);  // sorted: UP: room for (R, K)
 cudaError_t experts_tc(const ExpertParams &p, bool up, cudaStream_t s, int *rc);  // tcgen05 form, many rows
 
 }  // namespace nckv

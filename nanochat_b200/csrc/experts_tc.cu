@@ -1,4 +1,5 @@
-// The experts' products for many rows, on the tensor cores (tcgen05, accumulators in tensor memory).
+// The experts' products for many rows, on the tensor cores (tcgen05, accumulators in tensor memory).  The largest take the form on pairs of
+// CTAs (experts_pair.cu).
 //
 // Persistent CTAs, one per SM, walk over the tiles of all experts: 128 of an expert's sorted positions by BN
 // weight rows (UP: BN / 2 gate and the BN / 2 up rows of the same channels, so that a thread holds both
@@ -329,20 +330,25 @@ static cudaError_t et_launch(const ExpertParams &p, cudaStream_t s, int *rc) {
     return cudaGetLastError();
 }
 
+long long experts_tc_waves(bool up, int R, int E, int N, int bn) {
+    const long long m_tiles = R / ET_M + (E + 1) / 2;
+    const int per = up ? bn / 2 : bn;
+    return (m_tiles * ((N + per - 1) / per) + sm_count() - 1) / sm_count();
+}
+
+// Narrow tiles read the operands more often, but leave smaller last waves: take them where that wins
+// at an even spread of the positions.
+bool experts_tc_wide(bool up, int R, int E, int N) {
+    return 2 * experts_tc_waves(up, R, E, N, 256) * 10 <= experts_tc_waves(up, R, E, N, 128) * 11;
+}
+
 cudaError_t experts_tc(const ExpertParams &p, bool up, cudaStream_t s, int *rc) {
     if (p.E > ET_MAX_EXPERTS) {
         set_error("experts: at most %d experts", ET_MAX_EXPERTS);
         *rc = NCKV_E_UNSUPPORTED;
         return cudaSuccess;
     }
-    // Narrow tiles read the operands more often, but leave smaller last waves: take them where that wins
-    // at an even spread of the positions.
-    const long long m_tiles = p.R / ET_M + (p.E + 1) / 2;
-    auto waves = [&](int bn) {
-        const int per = up ? bn / 2 : bn;
-        return (m_tiles * ((p.N + per - 1) / per) + sm_count() - 1) / sm_count();
-    };
-    const bool wide = 2 * waves(256) * 10 <= waves(128) * 11;
+    const bool wide = experts_tc_wide(up, p.R, p.E, p.N);
     if (up) return wide ? et_launch<true, 256>(p, s, rc) : et_launch<true, 128>(p, s, rc);
     return wide ? et_launch<false, 256>(p, s, rc) : et_launch<false, 128>(p, s, rc);
 }

@@ -499,9 +499,11 @@ def expert_product(a, w, routing, up):
     if a.shape != (rows if up else routing.pairs, K) or E != routing.experts or a.dtype != w.dtype or not (a.is_contiguous() and w.is_contiguous()):
         raise RuntimeError(f"nckv::{name}: a {tuple(a.shape)} does not fit w {tuple(w.shape)} and {routing.pairs} pairs")
     out = torch.empty((routing.pairs, N) if up else (rows, routing.top, N), dtype=a.dtype, device=a.device)
-    ws = ops.workspace(a.device, 1, 1, 1)
+    ws, f32 = ops.workspace(a.device, 1, 1, 1), int(a.dtype == torch.float32)
+    need = _lib.lib.nckv_experts_workspace_bytes(int(up), routing.pairs, E, N, K, f32)
+    scratch = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
     idx, stream = _ctx(a)
     with ops._device_guard(idx):
-        _lib.call("nckv_experts", _ptr(a), _ptr(w), _ptr(out), _ptr(routing.offsets), _ptr(routing.slot), _ptr(routing.scale), int(up),
-                  routing.pairs, E, routing.top, N, K, int(a.dtype == torch.float32), _ptr(ws), stream)
+        _lib.call("nckv_experts_scratch", _ptr(a), _ptr(w), _ptr(out), _ptr(routing.offsets), _ptr(routing.slot), _ptr(routing.scale), int(up),
+                  routing.pairs, E, routing.top, N, K, f32, _ptr(scratch), need, _ptr(ws), stream)
     return out
