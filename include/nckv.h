@@ -332,6 +332,18 @@ NCKV_API int nckv_paged_fill(const void *src_k, const void *src_v, void *k_pool,
                     int n_jobs, int L, int Hkv, int D, int T_src, int page_tokens, int n_pages, void *stream);
 
 /*
+ * nckv_append_rope_norm and nckv_decode_attn (or their paged forms: block_table given, T_max the tokens of a page, batch_stride the
+ * distance between pages) of one new token per row in one launch, for few (row, kv head) pairs and short caches; nckv_decode_small_fits
+ * says which (capacity: tokens a row can hold).  q, k, v are the projections' outputs; strides of 0: packed rows.  The attention of a
+ * row that is not appended (NCKV_ST_OVERFLOW, NCKV_ST_BAD_SEQLEN) is zero.
+ */
+NCKV_API int nckv_decode_small_fits(int B, int Hq, int Hkv, int64_t capacity, int window_left);
+NCKV_API int nckv_decode_small(const void *q, const void *k, const void *v, int64_t q_stride, int64_t k_stride, int64_t v_stride, void *k_cache,
+                      void *v_cache, const int32_t *block_table, const int32_t *cache_seqlens, const void *cos, const void *sin, void *out,
+                      int B, int Hq, int Hkv, int D, int T_max, int max_pages, int n_pages, int64_t batch_stride, int64_t token_stride,
+                      int rope_len, int window_left, float qk_scale, float eps, int32_t *status, void *stream);
+
+/*
  * Dense (T_new >= 1) causal attention over a cache or plain k/v, tcgen05/TMEM tiles.
  * Replaces the full-causal and explicit-mask branches of _sdpa_attention
  * (flash_attention.py:79-80, 92-102) as reached from flash_attn_with_kvcache

@@ -57,6 +57,9 @@ SIGNATURES = {
     "nckv_decode_attn_paged": (c_int, [c_void_p] * 8 + [c_int] * 7 + [c_i64, c_i64, c_int, c_int, c_void_p, c_size_t,
                                                         c_void_p]),
     "nckv_paged_fill": (c_int, [c_void_p] * 5 + [c_int] * 7 + [c_void_p]),
+    "nckv_decode_small_fits": (c_int, [c_int] * 3 + [c_i64, c_int]),
+    "nckv_decode_small": (c_int, [c_void_p] * 3 + [c_i64] * 3 + [c_void_p] * 7 + [c_int] * 7 + [c_i64, c_i64, c_int, c_int, c_float, c_float,
+                                                                                               c_void_p, c_void_p]),
     "nckv_prefill_broadcast": (c_int, [c_void_p] * 5 + [c_int] * 7 + [c_void_p]),
     "nckv_prefill_attn": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_i64, c_i64, c_int, c_void_p, c_void_p]),
     "nckv_flash_attn_fwd": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_void_p]),

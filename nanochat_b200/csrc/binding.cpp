@@ -54,8 +54,8 @@ std::optional<Launch> launch_on(const c10::Device &dev, int B, int Hq, int Hkv) 
     return Launch{s, it->second};
 }
 
-// Append and attention of one layer, dense cache: nckv_append_rope_norm, then nckv_decode_attn (one new token per row)
-// or nckv_prefill_attn.  block_table: the caches are page pools (one new token per row).
+// Append and attention of one layer, dense cache: nckv_append_rope_norm, then nckv_decode_attn (one new token per row; few rows and short
+// caches: nckv_decode_small alone) or nckv_prefill_attn.  block_table: the caches are page pools (one new token per row).
 std::optional<Tensor> kv_attention(const Tensor &q, const Tensor &k, const Tensor &v, const Tensor &k_cache, const Tensor &v_cache,
                                    const std::optional<Tensor> &block_table, const Tensor &seqlens, const Tensor &cos, const Tensor &sin,
                                    int64_t window_left, double qk_scale, double eps) {
@@ -89,6 +89,17 @@ std::optional<Tensor> kv_attention(const Tensor &q, const Tensor &k, const Tenso
     const pybind11::gil_scoped_release unlocked;
     const c10::cuda::CUDAGuard guard(dev);
     const auto opt = q.options();
+    const int64_t pages = paged ? block_table->size(1) : 1;
+    if (T == 1 && nckv_decode_small_fits((int)B, (int)Hq, (int)Hkv, k_cache.size(1) * pages, (int)window_left)) {
+        Tensor y = at::empty({B, T, Hq, D}, opt);
+        if (nckv_decode_small(q.data_ptr(), k.data_ptr(), v.data_ptr(), sq, sk, sv, k_cache.data_ptr(), v_cache.data_ptr(),
+                              paged ? static_cast<const int32_t *>(block_table->data_ptr()) : nullptr, static_cast<const int32_t *>(seqlens.data_ptr()),
+                              cos.data_ptr(), sin.data_ptr(), y.data_ptr(), (int)B, (int)Hq, (int)Hkv, (int)D, (int)k_cache.size(1), (int)pages,
+                              (int)k_cache.size(0), k_cache.stride(0), k_cache.stride(1), (int)rope_len, (int)window_left, (float)qk_scale, (float)eps,
+                              static_cast<int32_t *>(on->ws.data_ptr()), on->stream) < 0)
+            return std::nullopt;
+        return y;
+    }
     Tensor q_rot = at::empty({B, T, Hq, D}, opt);
     int32_t *status = static_cast<int32_t *>(on->ws.data_ptr());
     const size_t ws_bytes = (size_t)on->ws.numel();

@@ -18,11 +18,11 @@ OUT = os.path.join(PKG, "libnckv.so")
 NATIVE = os.path.join(PKG, "_native.so")
 NATIVE_FOR = NATIVE + ".for"  # beside it: what it was built for
 BINDING = os.path.join(HERE, "binding.cpp")
-SOURCES = ["host.cu", "append.cu", "decode_attn.cu", "prefill_broadcast.cu", "lse_combine.cu",
+SOURCES = ["host.cu", "append.cu", "decode_attn.cu", "decode_small.cu", "prefill_broadcast.cu", "lse_combine.cu",
            "prefill_attn.cu", "p2p_exchange.cu", "glue.cu", "flash_attn_bwd.cu", "host_step.cu",
            "recurrent.cu", "recurrent_f32.cu", "norm_mix.cu", "window_attn.cu", "hyper_norm.cu",
            "gated_linear.cu", "delta.cu", "delta_chunk.cu", "experts.cu", "experts_tc.cu", "experts_pair.cu", "linear_cap.cu"]
-HEADERS = ["nckv_common.cuh", "vec_io.cuh", "tc05.cuh", "recurrent.cuh", "chunk.cuh", "experts.cuh", os.path.join("..", "..", "include", "nckv.h")]
+HEADERS = ["nckv_common.cuh", "vec_io.cuh", "tc05.cuh", "rope_row.cuh", "recurrent.cuh", "chunk.cuh", "experts.cuh", os.path.join("..", "..", "include", "nckv.h")]
 
 
 def _nvcc():

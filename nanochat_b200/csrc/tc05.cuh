@@ -56,6 +56,11 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+__device__ __forceinline__ uint32_t cluster_ctas() {
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
 __device__ __forceinline__ void cluster_sync() {  // all threads of the cluster
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

@@ -51,7 +51,7 @@ def compute_window_sizes(sequence_len, n_layer, window_pattern="SSSL"):
 
 
 def kv_attention(q, k, v, cos_sin_tables, window_size, kv_cache, layer_idx):
-    """The KV-cache branch of CausalSelfAttention.forward (gpt.py:97-121) in two launches.
+    """The KV-cache branch of CausalSelfAttention.forward (gpt.py:97-121) in two launches, or one (few rows, short caches).
 
     q: (B, T, Hq, D), k, v: (B, T, Hkv, D) straight from the projections (v already carries the
     value-embedding gate).  ``cos_sin_tables`` are the FULL tables (1, rope_len, 1, D/2): each row
@@ -68,7 +68,10 @@ def kv_attention(q, k, v, cos_sin_tables, window_size, kv_cache, layer_idx):
     left = int(window_size[0])
     left = left if left >= 0 else -1
     paged = getattr(kv_cache, "paged", False)
-    y = ops.append_and_attend(q, k, v, k_cache, v_cache, kv_cache.block_table if paged else None, seqlens, cos, sin, left)
+    call = (q, k, v, k_cache, v_cache, kv_cache.block_table if paged else None, seqlens, cos, sin, left)
+    y = ops.append_and_attend(*call)
+    if y is None and T == 1:
+        y = ops.append_and_attend_small(*call)
     if y is not None:
         if layer_idx == kv_cache.n_layers - 1:
             kv_cache.advance(T)

@@ -496,6 +496,45 @@ def append_and_attend(q, k, v, k_cache, v_cache, block_table, cache_seqlens, cos
     return _lib.native.kv_attention(q, k, v, k_cache, v_cache, block_table, cache_seqlens, cos, sin, window_left, QK_SCALE, RMS_EPS)
 
 
+def append_and_attend_small(q, k, v, k_cache, v_cache, block_table, cache_seqlens, cos, sin, window_left):
+    """Append and attention of one new token per row in one launch, for few rows and short caches (csrc/decode_small.cu); returns
+    (B, 1, Hq, D), or None where the single calls apply, which also say what they refuse."""
+    tensors = (q, k, v, k_cache, v_cache, cos, sin)
+    if any(not t.is_cuda or t.dtype != torch.bfloat16 or t.device != q.device for t in tensors) or any(t.dim() != 4 for t in tensors[:5]):
+        return None
+    B, T, Hq, D = q.shape
+    Hkv, paged = k.size(2), block_table is not None
+    if T != 1 or D != HEAD_DIM or B == 0 or Hkv == 0 or Hq % Hkv or k.shape != (B, 1, Hkv, D) or v.shape != k.shape or k_cache.shape != v_cache.shape or \
+            k_cache.stride() != v_cache.stride() or k_cache.shape[2:] != (Hkv, D) or k_cache.stride(3) != 1 or k_cache.stride(2) != D or \
+            cache_seqlens.dtype != torch.int32 or cache_seqlens.device != q.device or cache_seqlens.shape != (B,) or not cache_seqlens.is_contiguous() or \
+            cos.numel() != sin.numel() or cos.numel() == 0 or cos.numel() % (D // 2):
+        return None
+    if paged and (block_table.dtype != torch.int32 or block_table.device != q.device or block_table.dim() != 2 or block_table.size(0) != B or
+                  not block_table.is_contiguous() or k_cache.size(1) % PAGE_TILE):
+        return None
+    if not paged and k_cache.size(0) != B:
+        return None
+    pages = block_table.size(1) if paged else 1
+    with _device_guard(q.device.index):
+        if not _lib.lib.nckv_decode_small_fits(B, Hq, Hkv, k_cache.size(1) * pages, window_left):
+            return None
+    cos, sin = cos.reshape(-1, D // 2).contiguous(), sin.reshape(-1, D // 2).contiguous()
+    strides = [_token_stride(t) for t in (q, k, v)]
+    if None in strides:
+        q, k, v, strides = q.contiguous(), k.contiguous(), v.contiguous(), [0, 0, 0]
+    if any(t.data_ptr() % 16 for t in (q, k, v, k_cache, v_cache, cos, sin)) or k_cache.stride(0) % 8 or k_cache.stride(1) % 8 or \
+            k_cache.stride(1) < Hkv * D:
+        return None
+    y = torch.empty((B, 1, Hq, D), dtype=q.dtype, device=q.device)
+    idx, stream, ws = _launch_ctx(q, B, Hq, Hkv)
+    with _device_guard(idx):
+        _lib.call("nckv_decode_small", q.data_ptr(), k.data_ptr(), v.data_ptr(), *strides, k_cache.data_ptr(), v_cache.data_ptr(),
+                  block_table.data_ptr() if paged else None, cache_seqlens.data_ptr(), cos.data_ptr(), sin.data_ptr(), y.data_ptr(), B, Hq, Hkv, D,
+                  k_cache.size(1), pages, k_cache.size(0), k_cache.stride(0), k_cache.stride(1), cos.size(0), window_left, QK_SCALE, RMS_EPS,
+                  ws.data_ptr(), stream)
+    return y
+
+
 def decode_attention_split(q, k_cache, v_cache, cache_seqlens, split, part_out, part_lse, seqlen_offset=1,
                            peer_ptrs=None, step_counter=None):
     """One-token attention over this rank's block-cyclic part of the keys (``split = (world, rank,
