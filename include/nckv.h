@@ -301,6 +301,15 @@ NCKV_API int nckv_prefill_broadcast(const void *src_k, const void *src_v, void *
                            int T_dst, void *stream);
 
 /*
+ * The same without the host knowing the lengths.  prefill_note writes {src_seqlens[0], dst_seqlens[0]} to note (device) and to host_note
+ * (pinned host memory); prefill_broadcast_from copies note[0] tokens, nothing where note[1] is not 0 or note[0] is outside
+ * [0, min(T_src, T_dst)].  An event between the two tells the host while the copy runs.
+ */
+NCKV_API int nckv_prefill_note(const int32_t *src_seqlens, const int32_t *dst_seqlens, int32_t *note, int32_t *host_note, void *stream);
+NCKV_API int nckv_prefill_broadcast_from(const void *src_k, const void *src_v, void *dst_k, void *dst_v, int32_t *dst_seqlens, const int32_t *note,
+                                int L, int B, int Hkv, int D, int T_src, int T_dst, void *stream);
+
+/*
  * Paged KV storage (the "next" format after the dense (L, B, T_max, H, D) tensors of engine.py:98-100;
  * no counterpart in the reference).  One layer's K or V is a pool of pages (n_pages, page_tokens, Hkv,
  * D) with element strides (page_stride, token_stride, D, 1); block_table is int32 (B, max_pages): token t

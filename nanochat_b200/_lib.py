@@ -61,6 +61,8 @@ SIGNATURES = {
     "nckv_decode_small": (c_int, [c_void_p] * 3 + [c_i64] * 3 + [c_void_p] * 7 + [c_int] * 7 + [c_i64, c_i64, c_int, c_int, c_float, c_float,
                                                                                                c_void_p, c_void_p]),
     "nckv_prefill_broadcast": (c_int, [c_void_p] * 5 + [c_int] * 7 + [c_void_p]),
+    "nckv_prefill_note": (c_int, [c_void_p] * 5),
+    "nckv_prefill_broadcast_from": (c_int, [c_void_p] * 6 + [c_int] * 6 + [c_void_p]),
     "nckv_prefill_attn": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_i64, c_i64, c_int, c_void_p, c_void_p]),
     "nckv_flash_attn_fwd": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_void_p, c_void_p]),
     "nckv_flash_attn_bwd_workspace_bytes": (c_size_t, [c_int, c_int, c_int]),

@@ -62,15 +62,22 @@ class KVCache:
         """Broadcast a batch-1 prompt cache into every row of this (empty) cache (engine.py:123-137).
 
         Same preconditions as the reference: this cache is empty, layer/head/dim counts agree and
-        it is at least as long as ``other``.  One kernel launch copies K and V of all layers and
+        it is at least as long as ``other``.  One kernel copies K and V of all layers and
         sets ``cache_seqlens`` to the prompt length; ``prev_embedding`` is expanded to B rows.
         """
-        assert self.get_pos() == 0, "Cannot prefill a non-empty KV cache"
+        done = None
+        if self.n_layers == other.n_layers and self.n_heads == other.n_heads and self.head_dim == other.head_dim and \
+                self.max_seq_len >= other.max_seq_len and other.batch_size == 1 and not getattr(other, "paged", False):
+            # the copy is under way when the host learns the lengths; it did nothing where they do not allow it
+            done = ops.prefill_broadcast_from(other.k_cache, other.v_cache, other.cache_seqlens, self.k_cache, self.v_cache, self.cache_seqlens)
+        pos = done[0] if done else self.get_pos()
+        assert pos == 0, "Cannot prefill a non-empty KV cache"
         assert self.n_layers == other.n_layers and self.n_heads == other.n_heads and self.head_dim == other.head_dim
         assert self.max_seq_len >= other.max_seq_len
         assert other.batch_size == 1, "prefill broadcasts a batch-1 cache"
-        other_pos = other.get_pos()
-        ops.prefill_broadcast(other.k_cache, other.v_cache, self.k_cache, self.v_cache, self.cache_seqlens, other_pos)
+        other_pos = done[1] if done else other.get_pos()
+        if done is None or pos != 0 or not 0 <= other_pos <= other.k_cache.size(2):  # also what the single call refuses
+            ops.prefill_broadcast(other.k_cache, other.v_cache, self.k_cache, self.v_cache, self.cache_seqlens, other_pos)
         if other.prev_embedding is not None:
             self.prev_embedding = other.prev_embedding.expand(self.batch_size, -1, -1).clone()
 

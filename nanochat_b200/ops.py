@@ -625,6 +625,34 @@ def prefill_broadcast(src_k, src_v, dst_k, dst_v, dst_seqlens, p):
     _prefill_broadcast(src_k, src_v, dst_k, dst_v, dst_seqlens, p)
 
 
+def prefill_broadcast_from(src_k, src_v, src_seqlens, dst_k, dst_v, dst_seqlens):
+    """``prefill_broadcast`` of ``src_seqlens[0]`` tokens into a cache whose ``dst_seqlens[0]`` is 0, without the GPU waiting for the host: returns
+    (dst_seqlens[0], src_seqlens[0]) as they were.  Nothing is written where the first is not 0 or the second does not fit.  Returns None for
+    tensors that the single call has to look at."""
+    caches = (src_k, src_v, dst_k, dst_v)
+    dev = dst_k.device
+    if dev.type != "cuda" or any(t.device != dev or t.dim() != 5 or not t.is_contiguous() or t.dtype != dst_k.dtype or t.element_size() != 2 or
+                                 t.data_ptr() % 16 for t in caches) or src_k.shape != src_v.shape or dst_k.shape != dst_v.shape:
+        return None
+    L, B, T_dst, Hkv, D = dst_k.shape
+    T_src = src_k.size(2)
+    if src_k.shape != (L, 1, T_src, Hkv, D) or min(L, B, T_src, T_dst, Hkv, D) == 0 or D % 8 or any(
+            t.device != dev or t.dtype != torch.int32 or t.dim() != 1 or not t.is_contiguous() for t in (src_seqlens, dst_seqlens)) or \
+            src_seqlens.numel() != 1 or dst_seqlens.numel() != B:
+        return None
+    note, host_note = torch.empty(2, dtype=torch.int32, device=dev), torch.empty(2, dtype=torch.int32, pin_memory=True)
+    noted = torch.cuda.Event()
+    with torch.cuda.device(dev):
+        stream = _stream(dev)
+        _lib.call("nckv_prefill_note", _ptr(src_seqlens), _ptr(dst_seqlens), _ptr(note), _ptr(host_note), stream)
+        noted.record()
+        _lib.call("nckv_prefill_broadcast_from", _ptr(src_k), _ptr(src_v), _ptr(dst_k), _ptr(dst_v), _ptr(dst_seqlens), _ptr(note), L, B, Hkv, D,
+                  T_src, T_dst, stream)
+        noted.synchronize()
+    p, pos = host_note.tolist()
+    return pos, p
+
+
 def lse_combine(parts_o, parts_lse):
     """Merge partial attention results over disjoint key ranges; returns (bf16 out, fp32 lse)."""
     return _lse_combine(parts_o, parts_lse)
