@@ -540,6 +540,9 @@ NCKV_API int nckv_experts_scratch(const void *a, const void *w, void *out, const
                       int up, int R, int E, int top, int N, int K, int f32, void *workspace, size_t workspace_bytes, int32_t *status,
                       void *stream);
 
+/* out (rows, N) = silu(g) * u with [g; u] = w h, w (2 N, K) gate rows, then up rows, h (rows, K), bf16, K a multiple of 8, fp32 in between. */
+NCKV_API int nckv_gate_up(const void *h, const void *w, void *out, int rows, int N, int K, int32_t *status, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -102,6 +102,7 @@ SIGNATURES = {
     "nckv_route": (c_int, [c_void_p] * 4 + [c_int] * 3 + [c_void_p, c_size_t, c_void_p]),
     "nckv_experts": (c_int, [c_void_p] * 6 + [c_int] * 7 + [c_void_p, c_void_p]),
     "nckv_experts_workspace_bytes": (c_size_t, [c_int] * 6),
+    "nckv_gate_up": (c_int, [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 2),
     "nckv_experts_scratch": (c_int, [c_void_p] * 6 + [c_int] * 7 + [c_void_p, c_size_t, c_void_p, c_void_p]),
 }
 

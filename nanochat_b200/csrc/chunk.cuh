@@ -1,4 +1,4 @@
-// What the recurrences in chunks of 16 tokens share (delta_chunk.cu, recurrent_chunk.cu): m16n8k8 tf32 products of fp32 operands in
+// What a recurrence in chunks of 16 tokens needs (delta_chunk.cu): m16n8k8 tf32 products of fp32 operands in
 // two terms each, the sums over channels of pairs of tokens, the order of the operands in the records.
 #pragma once
 

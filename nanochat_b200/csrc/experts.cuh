@@ -15,8 +15,8 @@ struct ExpertParams {
     const void *a;         // UP: h (rows, K); else act (R, K)
     const void *w;         // UP: (E, 2 N, K) gate rows, then up rows; else (E, N, K)
     void *out;             // UP: act (R, N); else y (R, N) by slot
-    const int32_t *offsets, *slot;
-    const float *scale;
+    const int32_t *offsets, *slot;  // on pairs of CTAs without offsets: one expert with all R positions
+    const float *scale;             // there, null: 1
     int32_t *status;
     int R, E, top, N, K;
 };

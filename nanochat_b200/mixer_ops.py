@@ -115,6 +115,24 @@ def silu_mul(gate_up):
     return out
 
 
+# From here on the product with the activation in it; below, the library's smaller tiles fill the chip better (figures: csrc/experts_pair.cu).
+GATE_UP_ROWS, GATE_UP_VALUES = 1024, 1 << 21
+
+
+def gate_up(h, w):
+    """silu(gate) * up of the product with rows [gate; up] of ``w`` (2 N, K)."""
+    rows, K = h.shape
+    if rows < GATE_UP_ROWS or rows * (w.size(0) // 2) < GATE_UP_VALUES or not h.is_cuda or h.dtype != torch.bfloat16 or w.dtype != h.dtype or w.device != h.device or w.dim() != 2 or w.size(0) % 2 or \
+            w.size(1) != K or K % 8 or not (h.is_contiguous() and w.is_contiguous()) or (h.data_ptr() | w.data_ptr()) % 16:
+        return silu_mul(product(h, w))
+    out = torch.empty(rows, w.size(0) // 2, dtype=h.dtype, device=h.device)
+    status = ops.workspace(h.device, 1, 1, 1)
+    idx, stream = _ctx(h)
+    with ops._device_guard(idx):
+        _lib.call("nckv_gate_up", _ptr(h), _ptr(w), _ptr(out), rows, w.size(0) // 2, K, _ptr(status), stream)
+    return out
+
+
 def tanh_split(z, dtype):
     """tanh of fp32 rows (rows, R): float32 (rows, R), or bfloat16 (rows, 2 R) whose halves sum to it."""
     _check("tanh_split", z, dtypes=(torch.float32,))

@@ -267,7 +267,7 @@ class GatedFeedForward:
         self.w_down = weights["down"]
 
     def __call__(self, h):
-        return mo.product(mo.silu_mul(mo.product(h, self.w_in)), self.w_down)
+        return mo.product(mo.gate_up(h, self.w_in), self.w_down)
 
 
 class ShortConv:
