@@ -63,31 +63,42 @@ struct BwdParams {
     float scale, scale_log2;
 };
 
-// delta[b, h, t] = sum_c dO[b, t, h, c] * O[b, t, h, c]: half a warp per row, 16 bytes of each tensor per lane
+// delta[b, h, t] = sum_c dO[b, t, h, c] * O[b, t, h, c]: half a warp takes DELTA_ROWS rows, 16 bytes of each tensor per lane and row, all on
+// their way at once.  Bound by the bytes: 8 x 2048 tokens, 12 heads, 100 MB, a row at a time 22.3 us, now 18.3.
+constexpr int DELTA_ROWS = 4;
 __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const __nv_bfloat16 *out, const __nv_bfloat16 *dout,
                                                              float *delta, int B, int T, int Hq) {
-    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;  // (b, t, h) flattened
     const int j = threadIdx.x & 15;
-    const bool live = row < (long long)B * T * Hq;
-    float acc = 0.f;
-    if (live) {
-        const uint4 o = __ldg(reinterpret_cast<const uint4 *>(out + row * NCKV_D) + j);
-        const uint4 g = __ldg(reinterpret_cast<const uint4 *>(dout + row * NCKV_D) + j);
-        const __nv_bfloat162 *o2 = reinterpret_cast<const __nv_bfloat162 *>(&o);
-        const __nv_bfloat162 *g2 = reinterpret_cast<const __nv_bfloat162 *>(&g);
+    const long long rows = (long long)B * T * Hq, first = (long long)blockIdx.x * (16 * DELTA_ROWS) + (threadIdx.x >> 4);  // (b, t, h) flattened
+    uint4 o[DELTA_ROWS], g[DELTA_ROWS];
+#pragma unroll
+    for (int r = 0; r < DELTA_ROWS; ++r) {
+        const long long row = first + 16 * r;
+        o[r] = g[r] = make_uint4(0, 0, 0, 0);
+        if (row >= rows) continue;
+        o[r] = __ldg(reinterpret_cast<const uint4 *>(out + row * NCKV_D) + j);
+        g[r] = __ldg(reinterpret_cast<const uint4 *>(dout + row * NCKV_D) + j);
+    }
+    float mine = 0.f;  // lane r: row r
+#pragma unroll
+    for (int r = 0; r < DELTA_ROWS; ++r) {
+        const __nv_bfloat162 *o2 = reinterpret_cast<const __nv_bfloat162 *>(&o[r]);
+        const __nv_bfloat162 *g2 = reinterpret_cast<const __nv_bfloat162 *>(&g[r]);
+        float acc = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float2 a = __bfloat1622float2(o2[i]), c = __bfloat1622float2(g2[i]);
             acc += a.x * c.x + a.y * c.y;
         }
-    }
 #pragma unroll
-    for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (live && j == 0) {
-        const int h = (int)(row % Hq);
+        for (int off = 8; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if (j == r) mine = acc;
+    }
+    const long long row = first + 16 * j;
+    if (j < DELTA_ROWS && row < rows) {
         const long long bt = row / Hq;
-        const int t = (int)(bt % T), b = (int)(bt / T);
-        delta[((long long)b * Hq + h) * T + t] = acc;
+        const int h = (int)(row - bt * Hq), b = (int)(bt / T), t = (int)(bt - (long long)b * T);
+        delta[((long long)b * Hq + h) * T + t] = mine;
     }
 }
 
@@ -809,7 +820,7 @@ extern "C" int nckv_flash_attn_bwd(const void *q, const void *k, const void *v, 
     if (rc != NCKV_OK) return rc;
 
     const long long rows = (long long)B * T * Hq;
-    attn_bwd_delta_kernel<<<(unsigned)((rows + 15) / 16), 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(out),
+    attn_bwd_delta_kernel<<<(unsigned)((rows + 16 * DELTA_ROWS - 1) / (16 * DELTA_ROWS)), 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(out),
                                                                        static_cast<const __nv_bfloat16 *>(dout),
                                                                        static_cast<float *>(workspace), B, T, Hq);
     NCKV_CUDA_CHECK(cudaGetLastError());
