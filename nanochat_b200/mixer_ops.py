@@ -56,10 +56,10 @@ def product(a, w, f32_out=False):
 
 
 def add_product(y, a, w, y_scale=1.0, scale=1.0):
-    """y_scale * y + scale * (a @ w^T) in fp32 (y fp32)."""
+    """y <- y_scale * y + scale * (a @ w^T) in fp32 (y fp32, the caller's own: a result beside it costs a copy, 33 us for 16384 x 1536)."""
     if a.dtype == torch.bfloat16:
-        return torch.addmm(y, a, w.t(), out_dtype=torch.float32, beta=y_scale, alpha=scale)
-    return torch.addmm(y, a, w.t(), beta=y_scale, alpha=scale)
+        return torch.addmm(y, a, w.t(), out_dtype=torch.float32, beta=y_scale, alpha=scale, out=y)
+    return torch.addmm(y, a, w.t(), beta=y_scale, alpha=scale, out=y)
 
 
 def resid_norm(x, y, weight, eps, dtype, B, T, tokens=None, table=None, want_h=False, final_weight=None, mu=None,
