@@ -492,6 +492,12 @@ NCKV_API int nckv_recurrent(const void *q, const void *k, const void *v, int64_t
                       const void *gate, int64_t gate_stride, const float *norm_w, float eps, void *out, int64_t out_stride,
                       float *state, int B, int T, int H, int Dk, int Dv, int act_in, int f32, void *workspace,
                       size_t workspace_bytes, void *stream);
+/* the same; status (may be null) lets somewhat more heads than SMs take turns, which needs the workspace */
+NCKV_API int nckv_recurrent_status(const void *q, const void *k, const void *v, int64_t q_stride, int64_t k_stride, int64_t v_stride,
+                      const float *x, int64_t x_stride, const float *x0, const float *u, const float *decay,
+                      const void *gate, int64_t gate_stride, const float *norm_w, float eps, void *out, int64_t out_stride,
+                      float *state, int B, int T, int H, int Dk, int Dv, int act_in, int f32, void *workspace,
+                      size_t workspace_bytes, int32_t *status, void *stream);
 NCKV_API int nckv_gated_norm(const float *x, const void *gate, int64_t gate_stride, const float *w, void *out, int rows, int C,
                       int group, float eps, int gate_silu, int f32, void *stream);
 NCKV_API int nckv_resid_norm(const float *x, const void *y, int y_f32, const float *w, const int64_t *tokens, const void *table,

@@ -77,6 +77,8 @@ SIGNATURES = {
     "nckv_recurrent_workspace_bytes": (c_size_t, [c_int] * 5),
     "nckv_recurrent": (c_int, [c_void_p] * 3 + [c_i64] * 3 + [c_void_p, c_i64] + [c_void_p] * 4 +
                        [c_i64, c_void_p, c_float, c_void_p, c_i64, c_void_p] + [c_int] * 7 + [c_void_p, c_size_t, c_void_p]),
+    "nckv_recurrent_status": (c_int, [c_void_p] * 3 + [c_i64] * 3 + [c_void_p, c_i64] + [c_void_p] * 4 +
+                       [c_i64, c_void_p, c_float, c_void_p, c_i64, c_void_p] + [c_int] * 7 + [c_void_p, c_size_t, c_void_p, c_void_p]),
     "nckv_gated_norm": (c_int, [c_void_p, c_void_p, c_i64, c_void_p, c_void_p] + [c_int] * 3 + [c_float, c_int, c_int, c_void_p]),
     "nckv_resid_norm": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int] + [c_void_p] * 5 +
                         [c_int, c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p]),

@@ -164,6 +164,7 @@ size_t nckv_recurrent_workspace_bytes(int B, int T, int H, int Dk, int Dv) {
     using namespace nckv;
     if (B <= 0 || T <= 0 || H <= 0 || Dk <= 0 || Dv <= 0) return 0;
     const int n = rec_segments(T, B * H);
+    if (n == 1 && rec_turns(B * H, T)) return sizeof(int) * (size_t)B * H;
     return n == 1 ? 0 : sizeof(float) * (size_t)n * B * H * Dk * (Dv + 1);
 }
 
@@ -172,6 +173,15 @@ int nckv_recurrent(const void *q, const void *k, const void *v, int64_t q_stride
                    const void *gate, int64_t gate_stride, const float *norm_w, float eps, void *out, int64_t out_stride,
                    float *state, int B, int T, int H, int Dk, int Dv, int act_in, int f32, void *workspace,
                    size_t workspace_bytes, void *stream) {
+    return nckv_recurrent_status(q, k, v, q_stride, k_stride, v_stride, x, x_stride, x0, u, decay, gate, gate_stride, norm_w, eps, out, out_stride,
+                                 state, B, T, H, Dk, Dv, act_in, f32, workspace, workspace_bytes, nullptr, stream);
+}
+
+int nckv_recurrent_status(const void *q, const void *k, const void *v, int64_t q_stride, int64_t k_stride, int64_t v_stride,
+                          const float *x, int64_t x_stride, const float *x0, const float *u, const float *decay,
+                          const void *gate, int64_t gate_stride, const float *norm_w, float eps, void *out, int64_t out_stride,
+                          float *state, int B, int T, int H, int Dk, int Dv, int act_in, int f32, void *workspace,
+                          size_t workspace_bytes, int32_t *status, void *stream) {
     using namespace nckv;
     if (!q || !k || !v || !out || !state || (!x && !decay) || (x && (!x0 || !u)) || (norm_w && (!gate || !x))) {
         set_error("recurrent: null pointer argument");
@@ -195,6 +205,8 @@ int nckv_recurrent(const void *q, const void *k, const void *v, int64_t q_stride
     p.eps = eps; p.act_in = act_in;
     p.prod_out = nullptr; p.state_last = nullptr;
     p.C = 0; p.n_cols = 1;
+    p.status = status;
+    p.moved = status && workspace && !((uintptr_t)workspace & 3) && workspace_bytes >= sizeof(int) * (size_t)B * H ? static_cast<int *>(workspace) : nullptr;
     const uintptr_t elem = f32 ? 4 : 2;
     uintptr_t a = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)gate |
                   ((uintptr_t)(q_stride | k_stride | v_stride | gate_stride | Dk | Dv) * elem);
@@ -213,6 +225,7 @@ int nckv_recurrent(const void *q, const void *k, const void *v, int64_t q_stride
                   nckv_recurrent_workspace_bytes(B, T, H, Dk, Dv));
         return NCKV_E_CAPACITY;
     }
+    p.moved = nullptr;  // the workspace is the segments'
     const long long per_seg = (long long)B * H * Dk * Dv;
     float *states = static_cast<float *>(workspace), *prods = states + n_seg * per_seg;
     p.seg_len = (T + n_seg - 1) / n_seg;

@@ -60,6 +60,8 @@ struct RecurrentParams {
     int seg_len, n_seg;
     int n_cols;                       // column blocks per head (1 when gated)
     float eps;
+    int *moved;                       // room for turns (recurrent_turns_kernel), or null
+    int32_t *status;
     int act_in;                       // silu on q, k, v
     int vec;                          // all rows allow 4-element loads
 };
@@ -132,6 +134,19 @@ __device__ __forceinline__ Quad<float> load_quad(const float *p, bool in, int le
     }
     return r;
 }
+// the same past the SM's own cache: another SM may have left them
+template <bool VEC> __device__ __forceinline__ float4 load_kept(const float *p, bool in, int left) {
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (VEC) {
+        if (in) f = __ldcg(reinterpret_cast<const float4 *>(p));
+    } else if (in) {
+        f.x = __ldcg(p);
+        if (left > 1) f.y = __ldcg(p + 1);
+        if (left > 2) f.z = __ldcg(p + 2);
+        if (left > 3) f.w = __ldcg(p + 3);
+    }
+    return f;
+}
 template <bool VEC> __device__ __forceinline__ void store_quad(float *p, float4 a, int left) {
     if (VEC) {
         *reinterpret_cast<float4 *>(p) = a;
@@ -173,21 +188,28 @@ template <int BIT, int LEN> __device__ __forceinline__ int reduce_scatter(float 
     }
 }
 
-// CHANNEL: decay per token and key channel, bonus form.  OUT: false in the first pass over segments.
-template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC, int CL>
-__global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kernel(const RecurrentParams p) {
+// What the threads of a call share: one (row, head, column block) over tokens [t_begin, t_end).
+struct RecurrentShare {
+    int b, h, block, seg, t_begin, t_end;
+    const float *state_in;  // of the columns, null: zero
+    float *state_out;       // null: not kept
+};
+
+// CHANNEL: decay per token and key channel, bonus form.  OUT: false in the first pass over segments.  NT threads from tid 0 on, which meet at sync().
+template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC, int CL, typename Sync>
+__device__ __forceinline__ void recurrent_run(const RecurrentParams &p, const RecurrentShare &share, float *rec_smem, const int tid, const int NT,
+                                              const Sync &sync) {
     constexpr int TB = REC_BATCH, VG = 32 / KG, KP = 4 * KG * U, KQ = KP / 4, WC = CL * VG;  // WC: columns per warp
     constexpr int NB = KQ > 32 ? KQ / 32 : 1;                               // partial bonus sums per token
-    const int NT = blockDim.x, NW = NT >> 5;
+    const int NW = NT >> 5;
     const int VP = NW * WC, VQ = VP / 4;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, kg = lane % KG, vg = lane / KG;
-    const int h = blockIdx.x / p.n_cols, b = blockIdx.y, seg = blockIdx.z;
-    const int col0 = (blockIdx.x % p.n_cols) * VP, Dk = p.Dk, Dv = min(p.Dv - col0, VP);  // this CTA's columns of the head
+    const int warp = tid >> 5, lane = tid & 31, kg = lane % KG, vg = lane / KG;
+    const int h = share.h, b = share.b;
+    const int col0 = share.block * VP, Dk = p.Dk, Dv = min(p.Dv - col0, VP);  // this CTA's columns of the head
     const int C = p.C;
-    const int t_begin = seg * p.seg_len, t_end = min(p.T, t_begin + p.seg_len);
+    const int t_begin = share.t_begin, t_end = share.t_end;
     const bool gated = CHANNEL && OUT && p.norm_w != nullptr;
 
-    extern __shared__ __align__(16) float rec_smem[];
     // [x0 | u | norm weights], two buffers of [k | v | q | w | bonus], two output tiles
     const int per_buf = C * (KP + VP + (OUT ? KP : 0) + (CHANNEL ? KP : 0)) + (CHANNEL && OUT ? C * 4 : 0);
     float *s_x0 = rec_smem, *s_u = s_x0 + KP, *s_nw = s_u + KP, *s_buf = s_nw + VP, *s_out = s_buf + 2 * per_buf;
@@ -196,16 +218,15 @@ __global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kern
     // ---- this lane's part of the state: all loads in flight together ----------------------------------
     float2 S[U * 2][CL];  // [pair of key channels][column]
     const int v0 = warp * WC + vg * CL;
-    const long long state_base = (((long long)seg * p.B + b) * p.H + h) * (long long)Dk * p.Dv + col0;
     {
-        const float *src = p.state_in + state_base;
-        const bool have = p.state_in != nullptr;
+        const float *src = share.state_in;
+        const bool have = src != nullptr;
 #pragma unroll
         for (int i = 0; i < U * 4; ++i) {
             const int kc = (i >> 2) * 4 * KG + kg * 4 + (i & 3);
 #pragma unroll
             for (int c = 0; c < CL; c += 4) {
-                const float4 f = load_quad<VEC>(src + (long long)kc * p.Dv + v0 + c, have && kc < Dk && v0 + c < Dv, Dv - v0 - c).w;
+                const float4 f = load_kept<VEC>(src + (long long)kc * p.Dv + v0 + c, have && kc < Dk && v0 + c < Dv, Dv - v0 - c);
                 const float e[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -290,9 +311,9 @@ __global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kern
     }
     if (gated)
         for (int c = tid; c < VP; c += NT) s_nw[c] = c < Dv ? p.norm_w[h * p.Dv + c] : 0.f;
-    __syncthreads();
+    sync();
     stage(s_buf, min(C, t_end - t_begin));
-    __syncthreads();
+    sync();
 
     int parity = 0;
     for (int t0 = t_begin; t0 < t_end; t0 += C, parity ^= 1) {
@@ -375,7 +396,7 @@ __global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kern
             }
         }
         if (more) stage(s_buf + (parity ^ 1) * per_buf, min(C, t_end - t0 - C));
-        __syncthreads();
+        sync();
         if (OUT) {
             // 8 threads write a token; the buffers in use by the next chunk are the other ones
             for (int tb = 0; tb < n; tb += et_step) {  // the same trip count for all threads: the shuffles need whole warps
@@ -414,10 +435,8 @@ __global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kern
         }
     }
 
-    if (p.state_out) {
-        float *dst = p.state_last && seg == p.n_seg - 1
-                         ? p.state_last + ((long long)b * p.H + h) * Dk * p.Dv + col0
-                         : p.state_out + state_base;
+    if (share.state_out) {
+        float *dst = share.state_out;
 #pragma unroll
         for (int i = 0; i < U * 4; ++i) {
             const int kc = (i >> 2) * 4 * KG + kg * 4 + (i & 3);
@@ -432,12 +451,108 @@ __global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kern
         }
     }
     if (!OUT && p.prod_out && col0 == 0 && warp == 0 && vg == 0) {
-        float *dst = p.prod_out + (((long long)seg * p.B + b) * p.H + h) * Dk;
+        float *dst = p.prod_out + (((long long)share.seg * p.B + b) * p.H + h) * Dk;
 #pragma unroll
         for (int i = 0; i < U * 4; ++i) {
             const int kc = (i >> 2) * 4 * KG + kg * 4 + (i & 3);
             const float w = CHANNEL ? ((i & 1) ? prod2[i >> 1].y : prod2[i >> 1].x) : powf(w_head, (float)(t_end - t_begin));
             if (kc < Dk) dst[kc] = w;
+        }
+    }
+}
+
+template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC, int CL>
+__global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kernel(const RecurrentParams p) {
+    extern __shared__ __align__(16) float rec_smem[];
+    RecurrentShare s;
+    s.b = blockIdx.y; s.h = blockIdx.x / p.n_cols; s.block = blockIdx.x % p.n_cols; s.seg = blockIdx.z;
+    s.t_begin = s.seg * p.seg_len; s.t_end = min(p.T, s.t_begin + p.seg_len);
+    const int col0 = s.block * (blockDim.x >> 5) * CL * (32 / KG);
+    const long long head = (long long)s.b * p.H + s.h, per_head = (long long)p.Dk * p.Dv, per_seg = (long long)p.B * p.H * per_head;
+    s.state_in = p.state_in ? p.state_in + s.seg * per_seg + head * per_head + col0 : nullptr;
+    s.state_out = !p.state_out ? nullptr
+                               : (p.state_last && s.seg == p.n_seg - 1 ? p.state_last : p.state_out + s.seg * per_seg) + head * per_head + col0;
+    recurrent_run<T, KG, U, CHANNEL, OUT, VEC, CL>(p, s, rec_smem, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+}
+
+// Somewhat more heads than SMs.  With a CTA to a head some SMs hold two and the others one; one alone takes about 0.6 of the time of two side by
+// side, so the SMs with one are idle for the rest.  Here a CTA of two groups of warps stands on every SM, and the heads take turns: x SMs
+// hold two heads each (a) for 13/32 (constant decay: 3/8) of their tokens,
+// 2 x SMs one each (b) for the rest of theirs, which takes as long; then the b heads stand two
+// to an SM and the a heads alone.  A head that moves leaves its state in global memory and a flag; the rest of the heads stay where they are to the end.
+//   SM s < x:          heads 2 s and 2 s + 1, then 2 s alone
+//   SM x + j, j < 2 x: head 2 x + j, then, j odd, 2 x + j and 2 x + j - 1, j even, head j + 1
+// A head comes from a CTA with a lower index, so the waits end whatever part of the grid is resident.
+//   SM 3 x + j:        head 4 x + j
+// us, a CTA to a head / in turns, the same bits, B200: per channel, 24 heads of 64 x 64, 8 x 2048 tokens 537 / 471, 8 x 1024 275 / 247, 8 x 256 78 / 76; 7 x
+// 2048 537 / 467; constant, 12 heads of 64 x 128, 16 x 2048 861 / 682, 16 x 512 227 / 186, 13 x 1000 429 / 344.  Up to as many heads as SMs
+// 342 (8 x 2048); the parts' start and the registers of the second program cost some of what turns could give (419).
+struct RecurrentTurns {
+    int x, cut, cut_b;  // tokens of the first part of the a heads and of the b heads
+    int *moved;         // (B * H) zero: set when a head's state is there
+    int32_t *status;
+};
+template <typename T, int KG, int U, bool CHANNEL, bool VEC, int CL>
+__global__ void __launch_bounds__(512, 1) recurrent_turns_kernel(const RecurrentParams p, const RecurrentTurns r, int smem_floats) {
+    extern __shared__ __align__(16) float rec_smem[];
+    __shared__ RecurrentShare s_share[2];
+    __shared__ int s_there[2];
+    const int group = threadIdx.x >> 8, tid = threadIdx.x & 255, sm = blockIdx.x, j = sm - r.x;
+    const auto sync = [] { asm volatile("barrier.cta.sync %0, 256;" ::"r"((int)(threadIdx.x >> 8) + 1) : "memory"); };
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+        int head = -1, t0 = 0, t1 = p.T;
+        bool from = false, to = false;  // the head comes from another SM, goes to another one
+        if (sm < r.x) {
+            if (part == 0) {
+                head = 2 * sm + group; t1 = r.cut; to = group == 1;
+            } else if (group == 0) {
+                head = 2 * sm; t0 = r.cut;
+            }
+        } else if (j < 2 * r.x) {
+            if (part == 0) {
+                if (group == 0) { head = 2 * r.x + j; t1 = r.cut_b; to = !(j & 1); }
+            } else if (j & 1) {
+                head = 2 * r.x + j - group; t0 = r.cut_b; from = group == 1;
+            } else if (group == 0) {
+                head = j + 1; t0 = r.cut; from = true;
+            }
+        } else if (part == 0 && group == 0) {
+            head = r.x + sm;
+        }
+        if (head < 0) continue;  // uniform over the group
+        if (from) {
+            if (tid == 0) {
+                int there = 0;
+                const unsigned long long begin = global_timer_ns();
+                do {
+                    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(there) : "l"(r.moved + head) : "memory");
+                } while (!there && global_timer_ns() - begin < NCKV_WAIT_LIMIT_NS);
+                if (!there) atomicOr(r.status, (int)NCKV_ST_TIMEOUT);
+                s_there[group] = there;
+            }
+            sync();
+            if (!s_there[group]) return;
+        }
+        auto fill = [&](RecurrentShare &s) {
+            s.b = head / p.H; s.h = head - s.b * p.H; s.block = s.seg = 0;
+            s.t_begin = t0; s.t_end = t1;
+            s.state_out = p.state_out + (long long)head * p.Dk * p.Dv;
+            s.state_in = part == 0 ? p.state_in + (long long)head * p.Dk * p.Dv : s.state_out;
+        };
+        if constexpr (CHANNEL) {  // not in registers, of which there is none to spare (481 us, so 471; constant decay the other way round: 682, 729)
+            if (tid == 0) fill(s_share[group]);
+            sync();
+            recurrent_run<T, KG, U, CHANNEL, true, VEC, CL>(p, s_share[group], rec_smem + group * smem_floats, tid, 256, sync);
+        } else {
+            RecurrentShare s;
+            fill(s);
+            recurrent_run<T, KG, U, CHANNEL, true, VEC, CL>(p, s, rec_smem + group * smem_floats, tid, 256, sync);
+        }
+        sync();  // the next part uses the same shared memory, and the state is written
+        if (to && tid == 0) {
+            __threadfence();
+            asm volatile("st.release.gpu.global.s32 [%0], 1;" ::"l"(r.moved + head) : "memory");
         }
     }
 }
@@ -560,6 +675,13 @@ static cudaError_t rec_step_launch(RecurrentParams p, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// SMs with two heads at a time where heads take turns (recurrent_turns_kernel), 0: they do not.  Every head stands beside another one in one of the two parts at most.
+constexpr int REC_TURN_TOKENS = 256;  // 78 us / 76 there
+static int rec_turns(int pairs, int T) {
+    const int x = pairs - sm_count();
+    return T >= REC_TURN_TOKENS && x > 0 && 4LL * x <= pairs ? x : 0;
+}
+
 template <typename T, int KG, int U, bool CHANNEL, bool OUT, bool VEC, int CL = REC_LANE<U, CHANNEL>>
 static cudaError_t rec_launch_one(RecurrentParams p, cudaStream_t s) {
     constexpr int TB = REC_BATCH, WC = 32 * CL / KG, KP = 4 * KG * U;
@@ -581,6 +703,18 @@ static cudaError_t rec_launch_one(RecurrentParams p, cudaStream_t s) {
         const cudaError_t e = cudaFuncSetAttribute(recurrent_kernel<T, KG, U, CHANNEL, OUT, VEC, CL>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
+    }
+    if constexpr (OUT && VEC && sizeof(T) == 2 && KG == 16 && U == 1 && CL == REC_LANE<U, CHANNEL>) {
+        const int x = rec_turns(p.B * p.H, p.T);
+        if (x > 0 && p.moved && NT == 256 && p.n_cols == 1 && p.n_seg == 1 && 2 * smem <= 227 * 1024 - 16) {
+            cudaError_t e = cudaFuncSetAttribute(recurrent_turns_kernel<T, KG, U, CHANNEL, VEC, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * (int)smem);
+            if (e == cudaSuccess) e = cudaMemsetAsync(p.moved, 0, sizeof(int) * p.B * p.H, s);
+            if (e != cudaSuccess) return e;
+            const int cut = (int)((long long)p.T * (CHANNEL ? 13 : 12) / 32);
+            const RecurrentTurns r = {x, cut / C * C, (p.T - cut) / C * C, p.moved, p.status};
+            recurrent_turns_kernel<T, KG, U, CHANNEL, VEC, CL><<<sm_count(), 512, 2 * smem, s>>>(p, r, (int)(smem / sizeof(float)));
+            return cudaGetLastError();
+        }
     }
     recurrent_kernel<T, KG, U, CHANNEL, OUT, VEC, CL><<<dim3(p.H * p.n_cols, p.B, p.n_seg), NT, smem, s>>>(p);
     return cudaGetLastError();

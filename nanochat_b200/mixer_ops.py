@@ -338,11 +338,12 @@ def recurrent(q, k, v, state, B, T, heads, dim, vdim, decay=None, decay_logits=N
         ws = _scratch.get((idx, stream))
         if need and (ws is None or ws.numel() < need):
             ws = _scratch[(idx, stream)] = torch.empty(need, dtype=torch.uint8, device=q.device)
-        _lib.call("nckv_recurrent", _ptr(q), _ptr(k), _ptr(v), _row_stride(name, q), _row_stride(name, k), _row_stride(name, v),
+        _lib.call("nckv_recurrent_status", _ptr(q), _ptr(k), _ptr(v), _row_stride(name, q), _row_stride(name, k), _row_stride(name, v),
                   _ptr(decay_logits), _row_stride(name, decay_logits) if decay_logits is not None else 0, _ptr(decay_bias),
                   _ptr(bonus), _ptr(decay), _ptr(gate), _row_stride(name, gate) if gate is not None else 0,
                   _ptr(norm_weight), float(eps), _ptr(out), heads * vdim, _ptr(state), B, T, heads, dim, vdim,
-                  int(silu_inputs), int(q.dtype == torch.float32), _ptr(ws), ws.numel() if ws is not None else 0, stream)
+                  int(silu_inputs), int(q.dtype == torch.float32), _ptr(ws), ws.numel() if ws is not None else 0,
+                  _ptr(ops.workspace(q.device, 1, 1, 1)), stream)
     return out
 
 
