@@ -519,7 +519,8 @@ def expert_product(a, w, routing, up):
         raise RuntimeError(f"nckv::{name}: a {tuple(a.shape)} does not fit w {tuple(w.shape)} and {routing.pairs} pairs")
     out = torch.empty((routing.pairs, N) if up else (rows, routing.top, N), dtype=a.dtype, device=a.device)
     ws, f32 = ops.workspace(a.device, 1, 1, 1), int(a.dtype == torch.float32)
-    need = _lib.lib.nckv_experts_workspace_bytes(int(up), routing.pairs, E, N, K, f32)
+    # (few pairs never pay for the sorted copy, and the question costs a short prompt more than a microsecond)
+    need = _lib.lib.nckv_experts_workspace_bytes(1, routing.pairs, E, N, K, f32) if up and routing.pairs >= 256 else 0
     scratch = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
     idx, stream = _ctx(a)
     with ops._device_guard(idx):
