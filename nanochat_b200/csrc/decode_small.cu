@@ -2,7 +2,7 @@
 // append of k and v and the attention of one new token per row (append.cu and decode_attn.cu take three launches for it).
 //
 // With a handful of pairs the three launches' latencies and the host's time for them are all there is: 4 rows of 2 heads with some 64 keys took
-// 14 us a call (8.0 from a graph), all of it launches; now 9 to 11 (4.9), the host's time for one.  A cluster of CTAs takes a pair; its warps take
+// 14 us a call (8.0 from a graph), all of it launches; now 9 to 11 (5.1), the host's time for one.  A cluster of CTAs takes a pair; its warps take
 // the pair's keys 16 at a time, consecutive groups on different CTAs, on the grid of multiples of 16 (so a group lies in one page).  Every CTA
 // transforms the G query rows and the new key for itself while its first keys and values are on their way; the first CTA writes the new rows
 // into the cache.  No CTA reads a row that another one writes: the new token's key and value come from the inputs, as a group of their own.
@@ -10,7 +10,7 @@
 // A warp loads a group straight into the fragments of m16n8k16: a lane's 16-byte pieces of a key row are the channels of its places in two
 // steps of the sum (its order is free, q is arranged alike), a lane's 32 bytes of four value rows are turned into 16 columns' pairs with byte
 // permutes.  Two groups are on their way at once, all that a warp of an ordinary call has.  Eight warps to a CTA: with four of them, each with
-// twice the groups one after the other, 2000 keys of 12 heads took 9.4 us, now 7.5.  The warps' (max, sum, output) meet in shared memory
+// twice the groups one after the other, 2000 keys of 12 heads took 9.4 us, now 7.9.  The warps' (max, sum, output) meet in shared memory
 // (rows padded: unpadded, 16 heads to a kv head took 11.8 us for 2000 keys, now 10.1), the CTAs' through the cluster's.
 #include <math.h>
 
@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(DS_THREADS) decode_small_kernel(const DecodeSm
     __shared__ __align__(16) __nv_bfloat16 s_k[NCKV_D];
     __shared__ __align__(8) float s_ml[DS_WARPS][16][2];   // per warp and row: max (of base-2 logarithms), sum
     __shared__ __align__(8) float s_part[16][2];           // the CTA's
-    pdl_launch_dependents();
+    // No early release of what follows: an attention kernel behind the next append reads older cache rows before its own wait, and this
+    // grid's new row may be one of them.
     pdl_wait_prior_grids();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     const int ctas = (int)cluster_ctas(), rank = (int)cluster_rank(), pair = blockIdx.x / ctas, G = p.G;
@@ -343,11 +344,10 @@ static int small_clusters(bool ghi, int ctas) {
 
 // CTAs to a pair, 0: not taken.  As many as there are SMs for, all in one wave, and at most three groups of keys to a warp, where the other
 // kernels' single launches still cost more.  us from a CUDA graph, three launches / one, all keys present; a call by itself costs 13.9-15 / 8.5-11:
-//   1 x 2 + 2 heads: 100 keys 8.0 / 5.0, 2000 keys 9.2 / 7.2; 1 x 12 + 12 heads: 100 keys 8.4 / 5.0, 2000 keys 9.4 / 7.5, 3000 keys 10.4 / 8.8,
-//   4000 keys 10.2 / 10.4; 7 x 2 + 2: 4000 keys 10.6 / 10.4; 30 x 1 + 1: 2000 keys (four groups) 11.2 / 10.1; 18 x 8 + 1: 11.3 / 11.0;
-//   6 x 12 + 12: 500 keys 10.0 / 7.5; 8 x 16 + 16: 250 keys 10.5 / 7.2; 16 x 16 + 2: 1000 keys 11.1 / 8.4.
-// A group of more than 8 heads has twice the work: 1 x 16 + 1, 2000 keys 9.1 / 10.1 on clusters of 8, but 70 rows, 500 keys 23.0 / 10.4 and 140
-// rows, 250 keys 30.2 / 10.4.  Clusters of 8 that did not fit at once took 19 us for 2000 keys.
+//   4 x 2 + 2 heads: 64 keys 8.0 / 5.1, 2000 keys 8.9 / 7.4; 1 x 12 + 12 heads: 100 keys 8.4 / 5.5, 2000 keys 9.3 / 7.9, 3000 keys 10.4 / 9.0,
+//   four groups, 4000 keys, 10.2 / 10.8; 6 x 12 + 12: 500 keys 10.1 / 7.7; 8 x 16 + 16: 250 keys 10.5 / 7.8; 16 x 16 + 2: 1000 keys 11.1 / 8.8.
+// A group of more than 8 heads has twice the work: 1 x 16 + 1, 2000 keys 9.1 / 10.1 on clusters of 8, but 70 rows, 500 keys 23.0 / 10.9 and 140
+// rows, 250 keys 30.1 / 10.9.  Clusters of 8 that did not fit at once took 19 us for 2000 keys.
 static int small_ctas(int B, int Hq, int Hkv, long long capacity, int window_left) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || Hq / Hkv > DS_MAX_G) return 0;
     const long long pairs = (long long)B * Hkv, keys = window_left >= 0 && window_left + 1LL < capacity ? window_left + 1LL : capacity;
