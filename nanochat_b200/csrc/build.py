@@ -22,7 +22,7 @@ SOURCES = ["host.cu", "append.cu", "decode_attn.cu", "decode_small.cu", "prefill
            "prefill_attn.cu", "p2p_exchange.cu", "glue.cu", "flash_attn_bwd.cu", "host_step.cu",
            "recurrent.cu", "recurrent_f32.cu", "norm_mix.cu", "window_attn.cu", "hyper_norm.cu",
            "gated_linear.cu", "delta.cu", "delta_chunk.cu", "experts.cu", "experts_tc.cu", "experts_pair.cu", "linear_cap.cu"]
-HEADERS = ["nckv_common.cuh", "vec_io.cuh", "tc05.cuh", "rope_row.cuh", "recurrent.cuh", "chunk.cuh", "experts.cuh", os.path.join("..", "..", "include", "nckv.h")]
+HEADERS = ["nckv_common.cuh", "vec_io.cuh", "tc05.cuh", "rope_row.cuh", "recurrent.cuh", "experts.cuh", os.path.join("..", "..", "include", "nckv.h")]
 
 
 def _nvcc():
