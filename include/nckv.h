@@ -492,7 +492,8 @@ NCKV_API int nckv_recurrent(const void *q, const void *k, const void *v, int64_t
                       const void *gate, int64_t gate_stride, const float *norm_w, float eps, void *out, int64_t out_stride,
                       float *state, int B, int T, int H, int Dk, int Dv, int act_in, int f32, void *workspace,
                       size_t workspace_bytes, void *stream);
-/* the same; status (may be null) lets somewhat more heads than SMs take turns, which needs the workspace */
+/* the same; status (may be null) lets somewhat more heads than SMs take turns, which needs the workspace.  In either form the workspace is
+ * this call's alone until it has run. */
 NCKV_API int nckv_recurrent_status(const void *q, const void *k, const void *v, int64_t q_stride, int64_t k_stride, int64_t v_stride,
                       const float *x, int64_t x_stride, const float *x0, const float *u, const float *decay,
                       const void *gate, int64_t gate_stride, const float *norm_w, float eps, void *out, int64_t out_stride,

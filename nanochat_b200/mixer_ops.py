@@ -10,8 +10,6 @@ import torch
 
 from . import _lib, ops
 
-_scratch = {}  # (device index, stream) -> uint8 tensor for segmented recurrences
-
 
 def _check(name, *tensors, dtypes=(torch.bfloat16, torch.float32)):
     ops._require_cuda(name, *tensors)
@@ -335,14 +333,14 @@ def recurrent(q, k, v, state, B, T, heads, dim, vdim, decay=None, decay_logits=N
     idx, stream = _ctx(q)
     with ops._device_guard(idx):
         need = _lib.lib.nckv_recurrent_workspace_bytes(B, T, heads, dim, vdim)
-        ws = _scratch.get((idx, stream))
-        if need and (ws is None or ws.numel() < need):
-            ws = _scratch[(idx, stream)] = torch.empty(need, dtype=torch.uint8, device=q.device)
+        # segments' states, or the flags of heads that take turns: the call's own, or the graph's that holds it.  Shared by stream, two threads'
+        # calls would meet in it, and a replay would write to memory that a later, larger call has given back.
+        ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
         _lib.call("nckv_recurrent_status", _ptr(q), _ptr(k), _ptr(v), _row_stride(name, q), _row_stride(name, k), _row_stride(name, v),
                   _ptr(decay_logits), _row_stride(name, decay_logits) if decay_logits is not None else 0, _ptr(decay_bias),
                   _ptr(bonus), _ptr(decay), _ptr(gate), _row_stride(name, gate) if gate is not None else 0,
                   _ptr(norm_weight), float(eps), _ptr(out), heads * vdim, _ptr(state), B, T, heads, dim, vdim,
-                  int(silu_inputs), int(q.dtype == torch.float32), _ptr(ws), ws.numel() if ws is not None else 0,
+                  int(silu_inputs), int(q.dtype == torch.float32), _ptr(ws), need,
                   _ptr(ops.workspace(q.device, 1, 1, 1)), stream)
     return out
 
