@@ -482,14 +482,15 @@ __global__ void __launch_bounds__(REC_COLS / (32 * CL / KG) * 32) recurrent_kern
 // to an SM and the a heads alone.  A head that moves leaves its state in global memory and a flag; the rest of the heads stay where they are to the end.
 //   SM s < x:          heads 2 s and 2 s + 1, then 2 s alone
 //   SM x + j, j < 2 x: head 2 x + j, then, j odd, 2 x + j and 2 x + j - 1, j even, head j + 1
-// A head comes from a CTA with a lower index, so the waits end whatever part of the grid is resident.
 //   SM 3 x + j:        head 4 x + j
-// us, a CTA to a head / in turns, the same bits, B200: per channel, 24 heads of 64 x 64, 8 x 2048 tokens 537 / 471, 8 x 1024 275 / 247, 8 x 256 78 / 76; 7 x
-// 2048 537 / 467; constant, 12 heads of 64 x 128, 16 x 2048 861 / 682, 16 x 512 227 / 186, 13 x 1000 429 / 344.  Up to as many heads as SMs
-// 342 (8 x 2048); the parts' start and the registers of the second program cost some of what turns could give (419).
+// "SM" is a CTA's place in the order in which they start, taken from a counter: the order of their indices is promised nowhere.  A head comes from a
+// lower place, whose CTA has started and waits for nothing before it hands the head on, so the waits end whatever part of the grid is resident.
+// us, a CTA to a head / in turns, the same bits, B200: per channel, 24 heads of 64 x 64, 8 x 2048 tokens 537 / 475, 8 x 1024 275 / 246, 8 x 256 78 / 76;
+// constant, 12 heads of 64 x 128, 16 x 2048 861 / 689, 13 x 1000 429 / 346.  (By index instead of place 471, 245, 74, 684, 344.)  Up to as many
+// heads as SMs 342 (8 x 2048); the parts' start and the registers of the second program cost some of what turns could give (419).
 struct RecurrentTurns {
     int x, cut, cut_b;  // tokens of the first part of the a heads and of the b heads
-    int *moved;         // (B * H) zero: set when a head's state is there
+    int *moved;         // (B * H) zero: set when a head's state is there; the first, whose head never moves, counts the CTAs that have started
     int32_t *status;
 };
 template <typename T, int KG, int U, bool CHANNEL, bool VEC, int CL>
@@ -497,7 +498,11 @@ __global__ void __launch_bounds__(512, 1) recurrent_turns_kernel(const Recurrent
     extern __shared__ __align__(16) float rec_smem[];
     __shared__ RecurrentShare s_share[2];
     __shared__ int s_there[2];
-    const int group = threadIdx.x >> 8, tid = threadIdx.x & 255, sm = blockIdx.x, j = sm - r.x;
+    __shared__ unsigned s_place;
+    if (threadIdx.x == 0) s_place = (unsigned)atomicAdd(r.moved, 1);
+    __syncthreads();
+    const int group = threadIdx.x >> 8, tid = threadIdx.x & 255;
+    const int sm = (int)__reduce_max_sync(0xffffffffu, s_place), j = sm - r.x;  // (as one value of the warp: no register to spare for each lane's)
     const auto sync = [] { asm volatile("barrier.cta.sync %0, 256;" ::"r"((int)(threadIdx.x >> 8) + 1) : "memory"); };
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
@@ -540,7 +545,7 @@ __global__ void __launch_bounds__(512, 1) recurrent_turns_kernel(const Recurrent
             s.state_out = p.state_out + (long long)head * p.Dk * p.Dv;
             s.state_in = part == 0 ? p.state_in + (long long)head * p.Dk * p.Dv : s.state_out;
         };
-        if constexpr (CHANNEL) {  // not in registers, of which there is none to spare (481 us, so 471; constant decay the other way round: 682, 729)
+        if constexpr (CHANNEL) {  // not in registers, of which there is none to spare (10 us of 481; constant decay the other way round: 682 us, 729)
             if (tid == 0) fill(s_share[group]);
             sync();
             recurrent_run<T, KG, U, CHANNEL, true, VEC, CL>(p, s_share[group], rec_smem + group * smem_floats, tid, 256, sync);

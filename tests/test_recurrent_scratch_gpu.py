@@ -77,3 +77,21 @@ def test_replayed_behind_a_call_that_needs_more(form):
         assert all((t == 7).all() for t in others)
         side.synchronize()
     assert ops.read_status("cuda") == 0
+
+
+def test_heads_take_turns_while_other_kernels_hold_sms():
+    """Part of the grid is resident at first: whoever waits for a head, its CTA has started."""
+    run, S0 = inputs(SMS + SMS // 3, 256, 1, 64, 5)
+    S = S0.clone()
+    want = run(S)
+    a = torch.randn(8192, 8192, device="cuda").bfloat16()
+    b = a @ a
+    states, outs = [S0.clone() for _ in range(20)], []
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for _ in range(6):
+            torch.mm(a, a, out=b)
+    for s in states:
+        outs.append(run(s))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want) for o in outs) and all(torch.equal(s, S) for s in states) and ops.read_status("cuda") == 0
