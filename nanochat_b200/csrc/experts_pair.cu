@@ -45,10 +45,11 @@ struct EqCursor {
         if (e >= p.E) return false;
         const int tiles = s_first[e + 1] - s_first[e], local = idx - s_first[e] * n_tiles;
         m_hi = p.offsets ? p.offsets[e + 1] : p.R;
-        const int group = local / (eq_group(p.K) * n_tiles), in_group = local - group * eq_group(p.K) * n_tiles;
-        const int size = min(eq_group(p.K), tiles - group * eq_group(p.K));
+        const int most = min(eq_group(p.K), tiles);  // (so its product with n_tiles is not above the number of all tiles)
+        const int group = local / (most * n_tiles), in_group = local - group * most * n_tiles;
+        const int size = min(most, tiles - group * most);
         n = in_group / size;
-        m0 = (p.offsets ? p.offsets[e] : 0) + (group * eq_group(p.K) + in_group - n * size) * 2 * EQ_M;
+        m0 = (p.offsets ? p.offsets[e] : 0) + (group * most + in_group - n * size) * 2 * EQ_M;
         return true;
     }
 };

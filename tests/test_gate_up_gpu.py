@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from nanochat_b200 import _lib
 from nanochat_b200 import mixer_ops as mo
 from nanochat_b200 import ops
 
@@ -41,3 +42,18 @@ def test_rows_that_are_not_packed_and_other_types():
     assert torch.equal(mo.gate_up(h, w), mo.silu_mul(mo.product(h, w)))
     h, w = torch.randn(1024, 64, device="cuda"), torch.randn(4096, 64, device="cuda")
     assert torch.equal(mo.gate_up(h, w), mo.silu_mul(mo.product(h, w)))
+
+
+def test_so_many_weight_rows_that_a_group_of_tiles_had_no_number():
+    """A group is 65536 / K tiles of positions by all tiles of weights, 2^13 x 2^19 here; few positions leave it at their own tiles."""
+    rows, N, K = 3, 1 << 26, 8
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda", dtype=torch.bfloat16)
+    h, w, out = rand(rows, K), rand(2 * N, K), torch.zeros(rows, N, dtype=torch.bfloat16, device="cuda")
+    _lib.call("nckv_gate_up", h.data_ptr(), w.data_ptr(), out.data_ptr(), rows, N, K, ops.workspace(h.device, 1, 1, 1).data_ptr(),
+              torch.cuda.current_stream().cuda_stream)
+    assert ops.read_status("cuda") == 0
+    for at in range(0, N, 1 << 23):
+        part = slice(at, at + (1 << 23))
+        want, scale = wanted(h, torch.cat([w[:N][part], w[N:][part]]))
+        assert ((out[:, part].double() - want).abs() <= want.abs() / 256 + 1e-5 * scale * (1 + scale)).all()
