@@ -646,9 +646,11 @@ def prefill_broadcast_from(src_k, src_v, src_seqlens, dst_k, dst_v, dst_seqlens)
         stream = _stream(dev)
         _lib.call("nckv_prefill_note", _ptr(src_seqlens), _ptr(dst_seqlens), _ptr(note), _ptr(host_note), stream)
         noted.record()
-        _lib.call("nckv_prefill_broadcast_from", _ptr(src_k), _ptr(src_v), _ptr(dst_k), _ptr(dst_v), _ptr(dst_seqlens), _ptr(note), L, B, Hkv, D,
-                  T_src, T_dst, stream)
-        noted.synchronize()
+        try:
+            _lib.call("nckv_prefill_broadcast_from", _ptr(src_k), _ptr(src_v), _ptr(dst_k), _ptr(dst_v), _ptr(dst_seqlens), _ptr(note), L, B, Hkv, D,
+                      T_src, T_dst, stream)
+        finally:
+            noted.synchronize()  # also behind an error: until then host_note is the note's to write
     p, pos = host_note.tolist()
     return pos, p
 

@@ -49,3 +49,21 @@ def test_tensors_that_the_single_call_looks_at():
     assert ops.prefill_broadcast_from(src.k_cache, src.v_cache, src.cache_seqlens, strided, strided, dst.cache_seqlens) is None
     wide = torch.zeros(1, 3, 8, 2, 128, device="cuda")
     assert ops.prefill_broadcast_from(src.k_cache, src.v_cache, src.cache_seqlens, wide, wide, dst.cache_seqlens) is None
+
+
+def test_an_error_waits_for_the_note(monkeypatch):
+    """The pinned memory of the note goes back to its pool with the call, so nothing may still write to it."""
+    src, dst = caches(8, 8)
+    call = ops._lib.call
+
+    def failing(name, *args):
+        if name == "nckv_prefill_broadcast_from":
+            raise RuntimeError("planted")
+        return call(name, *args)
+
+    monkeypatch.setattr(ops._lib, "call", failing)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(int(0.2 * 1.9e9))  # the note waits behind it
+    with pytest.raises(RuntimeError, match="planted"):
+        dst.prefill(src)
+    assert torch.cuda.current_stream().query()
