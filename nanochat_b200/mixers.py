@@ -216,8 +216,8 @@ class ParallelMixer:
     def __call__(self, h, cache, B, T):
         lq, lk, lv, rq, rk, rv, rg = mo.product(h, self.w_in).split(self.widths, 1)
         y = mo.product(self.left.attend(lq, lk, lv, cache, B, T), self.left.w_o, f32_out=True)
-        return mo.add_product(y, self.right.attend(rq, rk, rv, rg, cache, B, T), self.right.w_o, self.left_scale,
-                              self.right_scale)
+        return mo.add_product_(y, self.right.attend(rq, rk, rv, rg, cache, B, T), self.right.w_o, self.left_scale,
+                               self.right_scale)
 
 
 class WkvMixer:
