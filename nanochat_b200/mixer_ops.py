@@ -528,7 +528,12 @@ def expert_product(a, w, routing, up):
     ws, f32 = ops.workspace(a.device, 1, 1, 1), int(a.dtype == torch.float32)
     # (few pairs never pay for the sorted copy, and the question costs a short prompt more than a microsecond)
     need = _lib.lib.nckv_experts_workspace_bytes(1, routing.pairs, E, N, K, f32) if up and routing.pairs >= 256 else 0
-    scratch = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
+    scratch = None
+    if need:
+        try:
+            scratch = torch.empty(need, dtype=torch.uint8, device=a.device)
+        except torch.OutOfMemoryError:  # the other form does without
+            need = 0
     idx, stream = _ctx(a)
     with ops._device_guard(idx):
         _lib.call("nckv_experts_scratch", _ptr(a), _ptr(w), _ptr(out), _ptr(routing.offsets), _ptr(routing.slot), _ptr(routing.scale), int(up),

@@ -61,3 +61,20 @@ def test_few_positions_take_the_other_form():
     for R, E, N, K in ((256, 16, 1024, 1536), (1024, 16, 1024, 1536), (6000, 16, 1024, 1536), (40000, 300, 1024, 1536), (24028, 16, 1024, 1532)):
         assert _lib.lib.nckv_experts_workspace_bytes(1, R, E, N, K, 0) == 0
     assert _lib.lib.nckv_experts_workspace_bytes(0, 24028, 16, 1536, 1024, 0) == 0 == _lib.lib.nckv_experts_workspace_bytes(1, 24028, 16, 1024, 1536, 1)
+
+
+def test_without_room_for_the_sorted_copy_the_other_form_answers(monkeypatch):
+    r = routed((640,) * 12)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    h, w = torch.randn(640 * 12, 1536, generator=gen, device="cuda").bfloat16(), torch.randn(12, 2048, 1536, generator=gen, device="cuda").bfloat16()
+    want, empty, need, refused = mo.expert_product(h, w, r, True), torch.empty, 2 * r.pairs * 1536, []
+
+    def short(*size, **kw):
+        if size == (need,) and kw.get("dtype") == torch.uint8:
+            refused.append(size)
+            raise torch.OutOfMemoryError("planted")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", short)
+    got = mo.expert_product(h, w, r, True)
+    assert refused and torch.equal(got, want) and ops.read_status("cuda") == 0
