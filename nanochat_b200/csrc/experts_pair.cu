@@ -335,7 +335,8 @@ cudaError_t experts_pair(ExpertParams p, bool up, void *sorted, cudaStream_t s, 
 
 }  // namespace nckv
 
-// The feed-forward's gate and up product with its activation: the up form with one expert that has all rows, in their order.  Against the
+// The feed-forward's gate and up product with its activation: the up form with one expert that has all rows, in their order (which sizes pay is the
+// caller's rule, gate_up_in_one).  Against the
 // library's product and an activation that reads its result (two halves, rounded between), B200, us: 1536 x 4096, 16384 rows 334 / 266, 4096 89 /
 // 68, 1024 25.4 / 21.4, 640 19.7 / 20.8, 300 11.4 / 14.0; 2048 x 5504, 16384 rows 575 / 483, 2048 79 / 64, 1024 41.9 / 36.3, 512 23.7 / 26.1;
 // 1024 x 2752, 4096 rows 52.6 / 33.3, 1024 15.7 / 16.2; 512 x 1024, 4096 rows 15.7 / 12.4, 2048 10.2 / 9.0, 1024 7.4 / 8.5; 256 x 512, 4096 rows 9.9

@@ -126,12 +126,33 @@ def silu_mul(gate_up):
 GATE_UP_ROWS, GATE_UP_VALUES = 1024, 1 << 21
 
 
+def gate_up_in_one(rows, values, channels, sms):
+    """Whether the activation pays inside the product: rows by ``values`` results of ``channels`` channels, in tiles of 256 x 128 on pairs of SMs.
+    What stands empty of its rounds of tiles, ragged ones too, costs it products; the library's smaller tiles leave less, but its pass behind the product
+    weighs less the more channels there are.  us, in one launch / in two, B200, by share filled: 512 channels 0.53 18.4 / 17.4, 0.58 18.4 / 21.5; 1024
+    0.58 34.8 / 29.7, 0.63 22.5 / 25.5; 1536 0.59 26.6 / 25.5, 0.64 26.6 / 29.6; 2048 0.46 32.8 / 27.7, 0.59 37.8 / 33.7, 0.68 49.3 / 52.2; 4096 0.52 59.5 / 44.0,
+    0.68 102 / 97, 0.80 62.4 / 66.3; 8192 0.71 246 / 204, 0.85 418 / 397, 0.90 266 / 283.  Of 408 sizes 8 lose, 4 percent at most; without
+    the line 54 did, up to 28 percent.  Twice an odd
+    number of results is a width for which the library is slow: 3453 results of 4096 channels 92 / 355."""
+    if rows < GATE_UP_ROWS or rows * values < GATE_UP_VALUES:
+        return False
+    rounds = -(-(-(-rows // 256) * -(-values // 128)) // (sms // 2))
+    return values % 4 != 0 or channels < 256 or rows * values >= min(0.86, 0.53 + channels / 15000) * rounds * (sms // 2) * 256 * 128
+
+
 def gate_up(h, w):
     """silu(gate) * up of the product with rows [gate; up] of ``w`` (2 N, K)."""
     rows, K = h.shape
     if rows < GATE_UP_ROWS or rows * (w.size(0) // 2) < GATE_UP_VALUES or not h.is_cuda or h.dtype != torch.bfloat16 or w.dtype != h.dtype or w.device != h.device or w.dim() != 2 or w.size(0) % 2 or \
-            w.size(1) != K or K % 8 or not (h.is_contiguous() and w.is_contiguous()) or (h.data_ptr() | w.data_ptr()) % 16:
+            w.size(1) != K or K % 8 or not (h.is_contiguous() and w.is_contiguous()) or (h.data_ptr() | w.data_ptr()) % 16 or \
+            not gate_up_in_one(rows, w.size(0) // 2, K, torch.cuda.get_device_properties(h.device).multi_processor_count):
         return silu_mul(product(h, w))
+    return gate_up_product(h, w)
+
+
+def gate_up_product(h, w):
+    """The same in one launch: packed bf16 h (rows, K) and w (2 N, K), K a multiple of 8."""
+    rows, K = h.shape
     out = torch.empty(rows, w.size(0) // 2, dtype=h.dtype, device=h.device)
     status = ops.workspace(h.device, 1, 1, 1)
     idx, stream = _ctx(h)

@@ -21,18 +21,24 @@ def test_against_64_bits(rows, N, K):
     rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
     h, w = rand(rows, K).bfloat16(), (rand(2 * N, K) * K ** -0.5).bfloat16()
     assert rows >= mo.GATE_UP_ROWS and rows * N >= mo.GATE_UP_VALUES
-    got, (want, scale) = mo.gate_up(h, w), wanted(h, w)
+    got, (want, scale) = mo.gate_up_product(h, w), wanted(h, w)
     # one rounding to the 8 bits of bf16 (at most 2^-8 of the value), fp32 sums of up to 8192 terms of about K^-1/2 and the activation
     assert ((got.double() - want).abs() <= want.abs() / 256 + 1e-5 * scale * (1 + scale)).all()
     assert ops.read_status("cuda") == 0
 
 
-@pytest.mark.parametrize("rows,N,K", [(1023, 4096, 64), (1024, 2047, 64), (3, 64, 64), (1100, 2048, 63)])
+@pytest.mark.parametrize("rows,N,K", [(1023, 4096, 64), (1024, 2047, 64), (3, 64, 64), (1100, 2048, 63), (1537, 1376, 4096), (1100, 2048, 2048)])
 def test_the_rest_takes_two_launches(rows, N, K):
     gen = torch.Generator(device="cuda").manual_seed(rows)
     rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
     h, w = rand(rows, K).bfloat16(), (rand(2 * N, K) * K ** -0.5).bfloat16()
     assert torch.equal(mo.gate_up(h, w), mo.silu_mul(mo.product(h, w)))
+
+
+def test_the_largest_take_one():
+    h, w = torch.randn(2048, 1536, device="cuda").bfloat16(), (torch.randn(8192, 1536, device="cuda") / 40).bfloat16()
+    got = mo.gate_up(h, w)
+    assert torch.equal(got, mo.gate_up_product(h, w)) and not torch.equal(got, mo.silu_mul(mo.product(h, w)))
 
 
 def test_rows_that_are_not_packed_and_other_types():
