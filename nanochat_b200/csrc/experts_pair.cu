@@ -313,9 +313,14 @@ template <bool UP> static cudaError_t eq_launch(const ExpertParams &p, cudaStrea
 // us, 16 experts, 4 a token, other form / pairs, B200: 1536 x 1024 up 6007 tokens 153.6 / 117.7, 16384 385 / 308, 1024 73.7 / 48.1, 384
 // 43.0 / 40.0, and the other way 1500 57.4 / 58.4, 256 34.8 / 39.9; down 6007 68.4 / 60.3, 1500 35.8 / 32.8, 1024 30.7 / 32.8; 2048 x
 // 1376 up 6007 251.9 / 199.7, 512 59.4 / 62.5, down 118.8 / 100.4, 1500 49.2 / 51.2.  The bits are the same.
+// The results of a tile of the down product take the time of some ten steps, in either form: with fewer steps they are the bound, and the other form's
+// tiles, half as large, fill the chip better.  us, other form / pairs: 512 channels, 16 experts, 1536 results 17584 positions 32.5 / 37.2, 41848 64.1 / 66.5;
+// 8 experts, 2048 results 2894 positions 13.6 / 14.9; 640 channels, 64 experts, 1024 results 21872 positions 42.5 / 45.0; 768 channels, 16 experts, 2048
+// results 12064 positions 48.9 / 45.3.  Of 35 sizes of up to 640 channels pairs lost in 28, of 110 of more in 9.
+constexpr int EQ_SHORT = 10;
 bool experts_in_pairs(bool up, int R, int E, int N, int K) {
-    if (E > EQ_MAX_EXPERTS || (!up && R <= 256LL * E)) return false;
     const int per = up ? EQ_BN / 2 : EQ_BN, steps = (K + EQ_K - 1) / EQ_K;
+    if (E > EQ_MAX_EXPERTS || (!up && (R <= 256LL * E || steps <= EQ_SHORT))) return false;
     const double m_tiles = std::max(R / (2. * EQ_M) + E / 2., (double)std::min(R, E));
     const double rounds = std::ceil(m_tiles * ((N + per - 1) / per) / (sm_count() / 2));
     const double pairs = up ? 64 * rounds + 100 * (8e-7 * R * K + 2) / (0.62 * steps) : 82 * rounds;
