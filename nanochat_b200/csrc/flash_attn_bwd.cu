@@ -63,16 +63,18 @@ struct BwdParams {
     float scale, scale_log2;
 };
 
-// delta[b, h, t] = sum_c dO[b, t, h, c] * O[b, t, h, c]: half a warp takes DELTA_ROWS rows, 16 bytes of each tensor per lane and row, all on
-// their way at once.  Bound by the bytes: 8 x 2048 tokens, 12 heads, 100 MB, a row at a time 22.3 us, now 18.3.
-constexpr int DELTA_ROWS = 4;
+// delta[b, h, t] = sum_c dO[b, t, h, c] * O[b, t, h, c]: half a warp takes ROWS rows, 16 bytes of each tensor per lane and row, all on their way
+// at once.  Four where the bytes are the bound, one where the time of a single warp is.  us, one / four, B200: 92 rows 2.8 / 4.9, 8192 3.8 / 5.4, 36864
+// 6.6 / 6.8, 49152 8.0 / 7.5, 196608 (8 x 2048 tokens, 12 heads, 100 MB) 21.9 / 19.0.
+constexpr long long DELTA_MANY = 40960;
+template <int ROWS>
 __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const __nv_bfloat16 *out, const __nv_bfloat16 *dout,
                                                              float *delta, int B, int T, int Hq) {
     const int j = threadIdx.x & 15;
-    const long long rows = (long long)B * T * Hq, first = (long long)blockIdx.x * (16 * DELTA_ROWS) + (threadIdx.x >> 4);  // (b, t, h) flattened
-    uint4 o[DELTA_ROWS], g[DELTA_ROWS];
+    const long long rows = (long long)B * T * Hq, first = (long long)blockIdx.x * (16 * ROWS) + (threadIdx.x >> 4);  // (b, t, h) flattened
+    uint4 o[ROWS], g[ROWS];
 #pragma unroll
-    for (int r = 0; r < DELTA_ROWS; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const long long row = first + 16 * r;
         o[r] = g[r] = make_uint4(0, 0, 0, 0);
         if (row >= rows) continue;
@@ -81,7 +83,7 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const __nv_bfloat16
     }
     float mine = 0.f;  // lane r: row r
 #pragma unroll
-    for (int r = 0; r < DELTA_ROWS; ++r) {
+    for (int r = 0; r < ROWS; ++r) {
         const __nv_bfloat162 *o2 = reinterpret_cast<const __nv_bfloat162 *>(&o[r]);
         const __nv_bfloat162 *g2 = reinterpret_cast<const __nv_bfloat162 *>(&g[r]);
         float acc = 0.f;
@@ -95,7 +97,7 @@ __global__ void __launch_bounds__(256) attn_bwd_delta_kernel(const __nv_bfloat16
         if (j == r) mine = acc;
     }
     const long long row = first + 16 * j;
-    if (j < DELTA_ROWS && row < rows) {
+    if (j < ROWS && row < rows) {
         const long long bt = row / Hq;
         const int h = (int)(row - bt * Hq), b = (int)(bt / T), t = (int)(bt - (long long)b * T);
         delta[((long long)b * Hq + h) * T + t] = mine;
@@ -820,9 +822,9 @@ extern "C" int nckv_flash_attn_bwd(const void *q, const void *k, const void *v, 
     if (rc != NCKV_OK) return rc;
 
     const long long rows = (long long)B * T * Hq;
-    attn_bwd_delta_kernel<<<(unsigned)((rows + 16 * DELTA_ROWS - 1) / (16 * DELTA_ROWS)), 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(out),
-                                                                       static_cast<const __nv_bfloat16 *>(dout),
-                                                                       static_cast<float *>(workspace), B, T, Hq);
+    const __nv_bfloat16 *o = static_cast<const __nv_bfloat16 *>(out), *d_o = static_cast<const __nv_bfloat16 *>(dout);
+    if (rows >= DELTA_MANY) attn_bwd_delta_kernel<4><<<(unsigned)((rows + 63) / 64), 256, 0, st>>>(o, d_o, static_cast<float *>(workspace), B, T, Hq);
+    else attn_bwd_delta_kernel<1><<<(unsigned)((rows + 15) / 16), 256, 0, st>>>(o, d_o, static_cast<float *>(workspace), B, T, Hq);
     NCKV_CUDA_CHECK(cudaGetLastError());
 
     static bool attr_set[64] = {false};  // per device; setting the attribute twice from racing threads is harmless
