@@ -123,3 +123,28 @@ def test_scores_of_minus_infinity_have_no_weight():
     y = ops.append_and_attend_small(q, k, v, kc, vc, None, seqlens, cos, sin, -1)[0, 0]
     want = attend(rotated, kc[0, 32:n + 1], vc[0, 32:n + 1], -1)
     assert (y.double() - want).abs().max() <= 1e-2 * want.abs().max()
+
+
+def test_steps_and_a_chunk_in_turn_on_the_same_rows():
+    """What a step leaves in the cache is what the next call, of whichever kernels, reads: beside a cache too long for the one launch."""
+    B, H, G, short, long = 3, 6, 2, 512, 16384
+    assert _lib.lib.nckv_decode_small_fits(B, H, G, short, -1) and not _lib.lib.nckv_decode_small_fits(B, H, G, long, -1)
+    cos, sin = precompute_rotary_embeddings(long, 128, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(BF)
+    caches = [KVCache(B, G, n, 128, 1, "cuda", BF) for n in (short, long)]
+    k0, v0 = rand(1, B, 200, G, 128), rand(1, B, 200, G, 128)
+    for c in caches:
+        c.k_cache[:, :, :200], c.v_cache[:, :, :200] = k0, v0
+        c.cache_seqlens.copy_(torch.tensor([30, 111, 200]))
+    for T in (1, 1, 1, 7, 1, 130, 1, 1):
+        q, k, v = rand(B, T, H, 128), rand(B, T, G, 128), rand(B, T, G, 128)
+        y, want = (kv_attention(q, k, v, (cos, sin), (-1, 0), c, 0) for c in caches)
+        # weights and outputs in bf16
+        assert (y.double() - want.double()).abs().max() <= 1e-2 * want.double().abs().max()
+    n = caches[0].cache_seqlens.tolist()
+    assert n == caches[1].cache_seqlens.tolist() == [30 + 143, 111 + 143, 200 + 143]
+    for b in range(B):
+        for a, c in zip((caches[0].k_cache, caches[0].v_cache), (caches[1].k_cache, caches[1].v_cache)):
+            assert torch.equal(a[0, b, :n[b]].view(torch.int16), c[0, b, :n[b]].view(torch.int16))
+    assert ops.read_status("cuda") == 0
