@@ -142,7 +142,6 @@ struct BuShared {  // behind the operand tiles of the dQ kernel
     // has been read".  (Every waiter has seen the phase before the one it waits for, so a parity stands for one phase only.)
     uint64_t bar_own, bar_last, bar_acc, bar_walk[BU_RING], bar_s[BU_BUFS], bar_p[BU_BUFS], bar_d[BU_RING];
     uint32_t tmem_slot;
-    int abort_flag;
 };
 constexpr int BU_SMEM_BYTES = 2 * BT_TILE_BYTES + BU_RING * 2 * BU_TILE_BYTES + (int)sizeof(BuShared);
 
@@ -177,7 +176,6 @@ struct BvShared {  // behind the operand tiles of the dK/dV kernel
     // are complete", bar_acc "its accumulators have been read"
     uint64_t bar_own, bar_last, bar_acc, bar_walk[BU_RING], bar_s[2], bar_p[2], bar_d[BU_RING];
     uint32_t tmem_slot;
-    int abort_flag;
     // the walked queries' values, one per accumulator column of a warp: -lse * log2(e) and delta / sqrt(D).  Every warp keeps
     // its own copy, so that the eight need not meet at a barrier in every unit
     alignas(16) float neg_lse2[BT_EW_THREADS / 32][BU / 2];
@@ -235,7 +233,6 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             mbar_init(&sh.bar_s[i], 1);
             mbar_init(&sh.bar_p[i], BT_EW_THREADS / 32);
         }
-        sh.abort_flag = 0;
         fence_mbar_init();
     }
     if (warp == 0) {
@@ -248,10 +245,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const uint32_t tmem_base = sh.tmem_slot;
     // unit u: S^T at columns 128 (u & 1) + [0, 64), dP^T at + [64, 128); dV at [256, 384), dK at [384, 512)
     const uint32_t tmem_dv = tmem_base + 256, tmem_dk = tmem_base + 384;
-    auto timed_out = [&]() {
-        sh.abort_flag = 1;
-        atomicOr(p.status, (int)NCKV_ST_TIMEOUT);
-    };
+    auto timed_out = [&]() { atomicOr(p.status, (int)NCKV_ST_TIMEOUT); };
 
     if (warp == BT_EW_THREADS / 32 + 1) {
         // =============== one thread issues the copies ================================================
@@ -540,7 +534,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             mbar_init(&sh.bar_s[i], 1);
             mbar_init(&sh.bar_p[i], BT_EW_THREADS / 32);
         }
-        sh.abort_flag = 0;
         fence_mbar_init();
     }
     if (warp == 0) {
@@ -553,10 +546,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const uint32_t tmem_base = sh.tmem_slot;
     // unit u: S at columns 128 (u % 3) + [0, 64), dP at + [64, 128); dQ at [384, 512)
     const uint32_t tmem_dq = tmem_base + 384;
-    auto timed_out = [&]() {
-        sh.abort_flag = 1;
-        atomicOr(p.status, (int)NCKV_ST_TIMEOUT);
-    };
+    auto timed_out = [&]() { atomicOr(p.status, (int)NCKV_ST_TIMEOUT); };
 
     if (warp == BT_EW_THREADS / 32 + 1) {
         // =============== one thread issues the copies ================================================
