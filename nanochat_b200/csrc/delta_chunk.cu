@@ -15,6 +15,10 @@
 //                                accumulator fragments: they are the left operand of the next chunk's products
 //                                as they stand (the order of the summed index is free), so no value crosses
 //                                lanes.  Records arrive by bulk copies through a ring in shared memory.
+//
+// The order of the sums stays: routers behind the rule choose among scores that nearly tie, and other last bits turn choices over.  A form with T and Q
+// multiplied into the rows ahead (two products on the chain from state to state, nearer to 64 bits) took 449 us where this one takes 644 (1 x 6007
+// tokens, 12 heads, both kernels), and 17 to 49 of a prompt's 6007 tokens took other experts in each layer behind it.
 #include "vec_io.cuh"
 
 namespace nckv {
@@ -85,7 +89,8 @@ __global__ void __launch_bounds__(KP, 640 / KP) delta_chunk_prepare_kernel(const
     for (int t = 0; t < DC_T; ++t) {
         part[t] = q[t] * q[t];
         part[DC_T + t] = k[t] * k[t];
-        // softplus in the fast functions: what it loses for very negative logits is far below one rounding of w
+        // softplus in the fast functions errs by 2^-21.4 (the logarithm) + 2^-24, so the argument by rate times that: some last places of w for rates of 1 and
+        // more, the same ones token after token where the decay is constant
         const float z = w[t] + x0;
         w[t] = on && t < n ? __expf(-rate * (fmaxf(z, 0.f) + __logf(1.f + __expf(-fabsf(z))))) : 1.f;
     }

@@ -41,7 +41,7 @@ struct LinearCapParams {
 // v / cap for two values, correctly rounded (to the bits of the division) where quotient and residue are normal numbers: the product with
 // the rounded reciprocal, corrected twice by its exact residue (Markstein's method; a uniform divisor leaves 2.5 instructions a value where
 // a division takes about ten and a check).  Values beyond 16 caps count as 16 caps, whose tanh is 1 too, so that an infinite one
-// leaves a quotient; what is no number stays none.
+// leaves a quotient; what is no number stays none.  (-0 would leave +0; a sum of products, which starts from +0, is never -0.)
 struct CapQuotient {
     float2 neg_cap, rcp;
     float most;

@@ -199,9 +199,10 @@ def cap_in_product(rows, words, channels, sms):
     """Whether the cap pays inside the product.  The library's product and the pass behind it take less where much of the last
     round of tiles of 256 x 256, or of the ragged tiles, is empty.  us, in one launch / in two, B200: 16384 x 32768 x 1536
     1294 / 1957, 6007 x 32768 x 2048 580 / 857, 1000 x 32768 x 1536 87 / 147, 2048 x 4096 x 1024 31 / 40, and the other
-    way 257 x 32768 x 1536 55 / 52 (half filled), 300 x 8192 x 1536 25 / 24 (one round, half filled).  Shorter channels (16384 x
-    32768 x 256 853 / 1330), single rounds (256 x 16384 x 2048 34 / 36) and 70 percent (1025 x 16384 x 1536 62 / 73) pay as well by
-    now; the lines lie where they did, for no model here has such heads."""
+    way 257 x 32768 x 1536 55 / 52 (half filled), 300 x 8192 x 1536 25 / 24 (one round, half filled), 300 x 32768 x 2048 64.5 / 62.4.  The lines are
+    wider than where the two cross: shorter channels (16384 x 32768 x 256 853 / 1330), single rounds (256 x 16384 x 2048 34 / 36) and two thirds filled
+    (200 x 32768 x 1536 40.9 / 46.0, 400 55.3 / 66.5, 600 71.7 / 95.2, 600 of 2048 channels 86 / 110) would pay in one launch too, which some 150 of the
+    numbers of rows below 776 have."""
     pairs = sms // 2
     rounds = -(-(-(-rows // 256) * -(-words // 256)) // pairs)
     return channels >= 1024 and rounds >= 2 and 4 * rows * words >= 3 * rounds * pairs * 256 * 256
